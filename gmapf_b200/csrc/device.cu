@@ -88,6 +88,8 @@ SearchParams search_params(Context& c) {
     Device& d = c.dev;
     SearchParams p{};
     p.rows = d.rows;
+    p.erow = d.erow;
+    p.third = d.third;
     p.cen = d.cen;
     p.n = c.map.n;
     p.req = d.req;
@@ -98,6 +100,8 @@ SearchParams search_params(Context& c) {
     p.K = c.K;
     p.rec = d.rec;
     p.epoch = d.epoch;
+    p.log = d.form != FORM_RECORDS ? d.log : nullptr;
+    p.queues = d.form == FORM_LOG_GLOBAL ? d.queues : nullptr;
     p.slots = d.slots;
     p.gbm = d.gbm;
     p.work_ctr = d.counters + CT_WORK;
@@ -227,48 +231,69 @@ int pick_slots(Context& c, int& blocks, std::string& err) {
     CK(cudaMemGetInfo(&freeb, &totalb));
     // the search state this context already holds counts as free: a reshape
     // reuses or replaces it
-    freeb += (size_t)d.rec_cap * (sizeof(Rec) * std::max(1, c.map.n) + sizeof(unsigned)) +
+    const int n = std::max(1, c.map.n);
+    freeb += (size_t)d.rec_cap * (sizeof(Rec) * n + sizeof(unsigned)) + (size_t)d.log_cap * sizeof(int4) * n +
              (size_t)d.gbm_cap * 4 * (size_t)d.bm_words;
     long long budget = c.opt.search_mem_budget > 0 ? c.opt.search_mem_budget : (40ll << 30);
     budget = std::min<long long>(budget, (long long)(freeb * 0.6));
-    const long long per_slot = (long long)std::max(1, c.map.n) * (long long)sizeof(Rec);
-    d.bm_words = search_bitmap_words(std::max(1, c.map.n));
+    d.bm_words = search_bitmap_words(n);
 
     // Candidates: visited placement (1 shared-memory bitmap, 2 stamped
     // records, 3 global bitmap, 4 global bitmap that a search at a batch's
-    // tail moves into its block's shared memory) and block size.  The
-    // score is the number of resident slots weighted by how close the claim
-    // check is: on chip x4, L2 x3, DRAM x2 (the record check misses L2 in
-    // every round); placement 4 wins a tie with placement 3 (a frame's tail
-    // then checks on chip).
+    // tail moves into its block's shared memory), block size and, on corridor
+    // maps, where the queues are.  The score is the number of resident slots
+    // weighted by how close the claim check is: on chip x4, L2 x3, DRAM x2 (the
+    // record check misses L2 in every round); placement 4 wins a tie with
+    // placement 3 (a frame's tail then checks on chip).  The kernel for
+    // corridor maps has placements 1 and 4; a slot with its bitmap on chip is
+    // worth 1.6 slots there (64x64 maze, 16,384 queries, T=32: 16 warps per SM
+    // on chip 2.94 ms, 24 with it in L2 3.0 ms; T=8: 14 on chip 8.4 ms, 24
+    // 8.2-8.6 ms), and the queues go to global memory where that gives 1.1
+    // times the slots (160x160 maze, T=32, C=16: 24 warps 16.5 ms, 20 warps with
+    // the queues in shared memory 18.9 ms; 64x64: 24 against 14 warps, 2.4 ms
+    // against 3.1).
     long long best_score = -1;
     int best_bt = 0;
     int best_vm = 2;
+    int best_form = FORM_RECORDS;
     long long best_slots = 0;
     const int want_vm = c.opt.visited_mode ? c.opt.visited_mode : c.tuned_vm;
     const int want_bt = c.opt.block_threads ? c.opt.block_threads : c.tuned_bt;
     for (int vm = 1; vm <= 4; vm++) {
         if (want_vm != 0 && want_vm != vm) continue;
-        const long long mem_slots = budget / (per_slot + (vm >= 3 ? 4ll * d.bm_words : 0));
         // the first of equal scores wins; placement 4 prefers 256-thread blocks
         // (measured faster than 128 on the 160x160 maze: 27.1 against 28.0 ms
         // for a frame batch)
         const int bts3[4] = {128, 64, 32, 256}, bts4[4] = {256, 128, 64, 32};
+        // corridor.cu's kernel, the longer the corridors the sooner: T = 32 on 8-,
+        // 12- and 24-cell mazes (84, 147 and 329 levels; 4,096 queries) 0.047,
+        // 0.080, 0.18 ms against search.cu's 0.059, 0.094, 0.24; T = 8 0.074,
+        // 0.20, 0.63 against 0.074, 0.20, 0.69; T = 4 0.135, 0.44, 1.21 against
+        // 0.120, 0.39, 1.25.  Between rectangles (8 to 49 levels) it is slower
+        // as soon as the fronts fill the lanes: T = 8, 1,313 triangles, 0.121
+        // against 0.096.
+        const bool log = (vm == 1 || vm == 4) && d.corridor_levels >= (c.T >= 16 ? 64 : 256);
         for (int bt : (vm == 4 ? bts4 : bts3)) {
             if (want_bt != 0 && bt != want_bt) continue;
             if (bt % c.T) continue;
-            const int per_sm = search_max_blocks_per_sm(c.T, c.C, bt, vm, d.bm_words);
-            if (per_sm <= 0) continue;
-            const int gpb = bt / 32;  // one request slot per warp
-            long long slots = std::min((long long)sms * per_sm * gpb, mem_slots);
-            slots = (slots / gpb) * gpb;
-            if (slots < gpb) continue;
-            const long long score = slots * (vm == 1 ? 4 : vm >= 3 ? 3 : 2) + (vm == 4 ? 1 : 0);
-            if (score > best_score) {
-                best_score = score;
-                best_bt = bt;
-                best_vm = vm;
-                best_slots = slots;
+            for (int form = log ? FORM_LOG : FORM_RECORDS; form <= (log ? FORM_LOG_GLOBAL : FORM_RECORDS); form++) {
+                const int per_sm = search_max_blocks_per_sm(c.T, c.C, bt, vm, d.bm_words, form);
+                if (per_sm <= 0) continue;
+                const int gpb = bt / 32;  // one request slot per warp
+                long long slots = std::min((long long)sms * per_sm * gpb,
+                                           budget / (long long)search_slot_bytes(n, vm, d.bm_words, form));
+                slots = (slots / gpb) * gpb;
+                if (slots < gpb) continue;
+                const long long weight = log ? (vm == 1 ? 64 : 40) : (vm == 1 ? 40 : vm >= 3 ? 30 : 20);
+                long long score = 10 * slots * weight + (vm == 4 ? 1 : 0);
+                if (form == FORM_LOG_GLOBAL) score = score * 9 / 10;
+                if (score > best_score) {
+                    best_score = score;
+                    best_bt = bt;
+                    best_vm = vm;
+                    best_form = form;
+                    best_slots = slots;
+                }
             }
         }
     }
@@ -279,10 +304,11 @@ int pick_slots(Context& c, int& blocks, std::string& err) {
     }
     c.block_threads = best_bt;
     d.vm = best_vm;
+    d.form = best_form;
     d.slots = (int)best_slots;
     blocks = (int)(best_slots / (best_bt / 32));
     // leave the kernel's shared-memory limit set for the chosen shape
-    search_max_blocks_per_sm(c.T, c.C, best_bt, best_vm, d.bm_words);
+    search_max_blocks_per_sm(c.T, c.C, best_bt, best_vm, d.bm_words, best_form);
     return GMAPF_OK;
 }
 
@@ -294,26 +320,45 @@ void release(Context& c, void* p) {
 }
 
 // Search state for the shape in c (T, C, visited placement, block size).
-// The record and bitmap arrays are kept while the new shape's slots fit
-// them (the autotuner reshapes a hundred times; a ~12 GB free, allocation
+// The record, log, queue and bitmap arrays are kept while the new shape's slots
+// fit them (the autotuner reshapes a hundred times; a ~12 GB free, allocation
 // and clear each time would take seconds).  Reuse needs no clearing: slot s
 // keeps its records together with its query epoch, so an old stamp never
-// equals a new epoch (modes 1 and 3 stamp 0, which no mode-2 epoch is), and
-// the bitmaps are cleared at the start of every query.
+// equals a new epoch (modes 1 and 3 stamp 0, which no mode-2 epoch is), a
+// search reads only the log and queue entries it wrote, and the bitmaps are
+// cleared at the start of every query.
 int alloc_search_state(Context& c, std::string& err) {
     Device& d = c.dev;
     int blocks = 0;
     int rc = pick_slots(c, blocks, err);
     if (rc) return rc;
-    if (!d.rec || d.slots > d.rec_cap) {
+    const size_t n = std::max(1, c.map.n);
+    if (d.form == FORM_RECORDS && (!d.rec || d.slots > d.rec_cap)) {
         release(c, d.rec);
         release(c, d.epoch);
         d.rec = nullptr;
         d.epoch = nullptr;
         d.rec_cap = 0;
-        DALLOC(d.rec, (size_t)d.slots * std::max(1, c.map.n));
+        DALLOC(d.rec, d.slots * n);
         DALLOC(d.epoch, (size_t)d.slots);
         d.rec_cap = d.slots;
+    }
+    if (d.form != FORM_RECORDS && (!d.log || d.slots > d.log_cap)) {
+        release(c, d.log);
+        d.log = nullptr;
+        d.log_cap = 0;
+        DALLOC(d.log, d.slots * n);
+        d.log_cap = d.slots;
+    }
+    if (d.form == FORM_LOG_GLOBAL) {
+        const size_t need = d.slots * corridor_queue_bytes(c.C, c.T);
+        if (need > d.queue_cap) {
+            release(c, d.queues);
+            d.queues = nullptr;
+            d.queue_cap = 0;
+            DALLOC(d.queues, need / sizeof(int));
+            d.queue_cap = need;
+        }
     }
     if (d.vm >= 3 && (!d.gbm || d.slots > d.gbm_cap)) {
         release(c, d.gbm);
@@ -323,6 +368,25 @@ int alloc_search_state(Context& c, std::string& err) {
         d.gbm_cap = d.slots;
     }
     return GMAPF_OK;
+}
+
+// after the shape is settled: the arrays of the other kernel's trials go
+void trim_search_state(Context& c) {
+    Device& d = c.dev;
+    if (d.form == FORM_RECORDS) {
+        release(c, d.log);
+        release(c, d.queues);
+        d.log = nullptr;
+        d.queues = nullptr;
+        d.log_cap = 0;
+        d.queue_cap = 0;
+    } else {
+        release(c, d.rec);
+        release(c, d.epoch);
+        d.rec = nullptr;
+        d.epoch = nullptr;
+        d.rec_cap = 0;
+    }
 }
 
 int search_blocks(Context& c) { return c.dev.slots / (c.block_threads / 32); }
@@ -424,7 +488,15 @@ int device_start(Context& c, std::string& err) {
     DALLOC(d.gstart, m.gstart.size());
     DALLOC(d.glist, m.glist.size());
     DALLOC(d.degen, m.degen.size());
-    CK(cudaMemcpy(d.rows, m.rows.data(), sizeof(SearchRow) * n, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(d.rows, m.rows.data(), sizeof(SearchRow) * n, cudaMemcpyHostToDevice, d.stream));
+    d.corridor_levels = corridor_levels(m, c.scenes);
+    if (d.corridor_levels >= 64) {
+        DALLOC(d.erow, 4 * (size_t)n);
+        DALLOC(d.third, n);
+        launch_edge_rows(d.stream, d.rows, n, d.erow, d.third);
+        CK(cudaGetLastError());
+    }
+    CK(cudaStreamSynchronize(d.stream));
     CK(cudaMemcpy(d.cen, m.cen.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d.tri, m.tri.data(), sizeof(float2) * 3 * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d.gstart, m.gstart.data(), sizeof(int) * m.gstart.size(), cudaMemcpyHostToDevice));
@@ -557,8 +629,11 @@ void device_free(Context& c) {
     d.allocs.clear();
     d.rec = nullptr;  // freed above: a later start allocates anew
     d.epoch = nullptr;
+    d.log = nullptr;
+    d.queues = nullptr;
+    d.queue_cap = 0;
     d.gbm = nullptr;
-    d.rec_cap = d.gbm_cap = 0;
+    d.rec_cap = d.log_cap = d.gbm_cap = 0;
     d.slots = 0;
     for (auto& e : d.ev)
         if (e) cudaEventDestroy(e), e = nullptr;
@@ -1066,8 +1141,8 @@ int device_autotune(Context& c, std::string& err) {
                 trial(T, C, vm, 0);
                 if (trials.size() == before) continue;  // shape does not fit this placement
                 if (vm == 4)
-                    vm4_fits = search_max_blocks_per_sm(T, C, c.block_threads, 4, d.bm_words) ==
-                               search_max_blocks_per_sm(T, C, c.block_threads, 3, d.bm_words);
+                    vm4_fits = search_max_blocks_per_sm(T, C, c.block_threads, 4, d.bm_words, d.form) >=
+                               search_max_blocks_per_sm(T, C, c.block_threads, 3, d.bm_words, FORM_RECORDS);
                 best_at_T = std::min(best_at_T, trials.back().ms);
                 const long long f = trials.back().found;
                 best_found_so_far = std::max(best_found_so_far, f);
@@ -1120,7 +1195,9 @@ int device_autotune(Context& c, std::string& err) {
     CK(cudaStreamSynchronize(d.stream));
     std::memset(c.h_stats, 0, sizeof(unsigned long long) * ST_COUNT);
     for (int k = 0; k < ST_COUNT; k++) c.stats_prev[k] = 0;
-    return device_reconfigure_search(c, err);
+    const int rc = device_reconfigure_search(c, err);
+    if (rc == GMAPF_OK) trim_search_state(c);
+    return rc;
 }
 
 }  // namespace gmapf_b200

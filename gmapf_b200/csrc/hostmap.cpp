@@ -167,6 +167,41 @@ static void bfs_hops(const HostMap& m, int src, std::vector<unsigned short>& d) 
     }
 }
 
+int corridor_levels(const HostMap& m, const std::vector<SceneInfo>& scenes) {
+    // levels and triangles of a breadth-first wave from each scene's first
+    // triangle or from the farthest one from it, whichever is longer
+    long long levels = 0, nodes = 0, waves = 0;
+    std::vector<int> d(m.n, -1), q;
+    for (const SceneInfo& si : scenes) {
+        if (si.n == 0) continue;
+        int src = si.node_base;
+        long long lv = 0, cnt = 0;
+        for (int pass = 0; pass < 2; pass++) {
+            for (int v : q) d[v] = -1;
+            q.assign(1, src);
+            d[src] = 0;
+            for (size_t h = 0; h < q.size(); h++) {
+                const SearchRow& r = m.rows[q[h]];
+                const int nb[3] = {r.n0, r.n1, r.n2};
+                for (int k = 0; k < r.deg; k++)
+                    if (d[nb[k]] < 0) {
+                        d[nb[k]] = d[q[h]] + 1;
+                        q.push_back(nb[k]);
+                    }
+            }
+            src = q.back();  // a farthest one
+            if (d[src] + 1 > lv) {
+                lv = d[src] + 1;
+                cnt = (long long)q.size();
+            }
+        }
+        levels += lv;
+        nodes += cnt;
+        waves++;
+    }
+    return waves > 0 && nodes <= 16 * levels ? (int)(levels / waves) : 0;
+}
+
 void landmark_distances(const HostMap& m, int count, std::vector<unsigned short>& out) {
     out.assign((size_t)count * std::max(0, m.n), 65535);
     if (m.n == 0 || count <= 0) return;

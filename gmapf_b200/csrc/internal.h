@@ -52,8 +52,27 @@ enum ErrBits {
     ERR_BAD_REQUEST = 8  // a request named a node outside the map
 };
 
+// What a search needs to expand node v reached through neighbour slot s of v
+// (the slot of its parent; s = 3: no parent, a search's root): the candidates
+// are v's neighbours other than the parent, in slot order, each as a directed
+// edge (node << 2 | its slot of v, 3 if it does not list v; -1: none) with its
+// centroid.  Row v << 2 | s; 32 bytes, one sector, read as a whole or by half.
+// A third candidate (rows with s = 3 only) is in a separate array.
+struct __align__(16) EdgeHalf {
+    int e;
+    unsigned info;  // its slot as a one-hot bit 0-2, kEdgeThird, and (first half) v's degree from bit 4
+    float x, y;
+};
+constexpr unsigned kEdgeThird = 8;  // (first half) there is a third candidate
+struct __align__(32) EdgeRow {
+    EdgeHalf x, y;
+};
+static_assert(sizeof(EdgeRow) == 32, "edge row layout");
+
 struct SearchParams {
     const SearchRow* rows;
+    const EdgeRow* erow;     // corridor maps (log set): 4 per node
+    const EdgeHalf* third;   // corridor maps: per node, the third candidate of its row 3
     const float2* cen;
     int n;
     const int4* req;         // {agent (or -1), start, target, output row}
@@ -63,6 +82,8 @@ struct SearchParams {
     float K;
     Rec* rec;                // slots * n
     unsigned* epoch;         // per slot
+    int4* log;               // corridor maps, instead of rec: slots * n, the claims of a slot's search in order
+    int* queues;             // corridor maps: slots x corridor_queue_bytes, or null (queues in shared memory)
     int slots;
     unsigned* gbm;           // visited mode 3: bm_words 32-bit words per slot, global
     int* work_ctr;
@@ -78,7 +99,7 @@ struct SearchParams {
     int* ag_path_len;
     unsigned long long* stats;  // ST_COUNT counters
     int* err;
-    // search state slots [slot_base, slot_base + slots) of rec/epoch/gbm
+    // search state slots [slot_base, slot_base + slots) of rec/epoch/log/queues/gbm
     int slot_base;
     // serving ring (ring_cap > 0): request r of this launch is query
     // q = ring_base + r, stored at req[q % ring_cap]; its completion word
@@ -173,6 +194,8 @@ void launch_collide_progress(cudaStream_t s, const MoverParams& p);
 void launch_funnel(cudaStream_t s, const MoverParams& p);
 void launch_prepare_batch(cudaStream_t s, const int* starts, const int* targets, int n, int nodes,
                           int4* req, int* req_count, int* work_ctr, int* err);
+// the 4 n edge rows of a map with the given search rows
+void launch_edge_rows(cudaStream_t s, const SearchRow* rows, int n, EdgeRow* out, EdgeHalf* third);
 // search.cu
 // persistent: groups pull requests from *work_ctr until *req_count_d is reached.
 // plain: one request per group, requests [base, base + groups).
@@ -181,9 +204,19 @@ void launch_prepare_batch(cudaStream_t s, const int* starts, const int* targets,
 // bitmap per slot in global memory (p.gbm, small enough to stay in L2).
 cudaError_t launch_search(cudaStream_t s, const SearchParams& p, int blocks, int block_threads,
                           bool persistent, int req_base, int vm, int bm_words);
+// which kernel a search runs on: search.cu's, with a record per claimed node,
+// or corridor.cu's, with a claim log, its queues in shared or in global memory
+enum SearchForm { FORM_RECORDS = 0, FORM_LOG, FORM_LOG_GLOBAL };
+// device memory of one request slot: records or claim log, and visited state
+size_t search_slot_bytes(int n_nodes, int vm, int bm_words, int form);
 size_t search_smem_bytes(int C, int block_threads, int bm_words, int T, int vm);
 int search_bitmap_words(int n_nodes);
-int search_max_blocks_per_sm(int T, int C, int block_threads, int vm, int bm_words);
+int search_max_blocks_per_sm(int T, int C, int block_threads, int vm, int bm_words, int form);
+// corridor.cu (launch_search goes there when p.log is set)
+cudaError_t launch_corridor_search(cudaStream_t s, const SearchParams& p, int blocks, int block_threads,
+                                   bool persistent, int req_base, int vm, int bm_words);
+int corridor_max_blocks_per_sm(int T, int C, int block_threads, int vm, int bm_words, bool queues_global);
+size_t corridor_queue_bytes(int C, int T);
 
 // ------------------------------------------------------------------- host --
 
@@ -220,6 +253,10 @@ void build_host_map(const gmapf_node* nodes, int n, HostMap& out);
 // global triangle ids; fills each scene's triangle range, bounds and
 // point-location grid (offsets into the concatenated grid arrays).
 void concat_host_maps(const std::vector<const HostMap*>& maps, HostMap& out, std::vector<SceneInfo>& scenes);
+// How long a map's corridors are: the levels of a breadth-first wave from a far
+// triangle (the mean over the scenes), 0 when the waves hold more than 16
+// triangles per level on average (open ground).
+int corridor_levels(const HostMap& m, const std::vector<SceneInfo>& scenes);
 // Hop distances from `count` landmark triangles chosen by farthest-point
 // sampling over the neighbour graph (unreachable: 65535), count * n values.
 void landmark_distances(const HostMap& m, int count, std::vector<unsigned short>& out);
@@ -237,6 +274,9 @@ struct Device {
     cudaStream_t stream = nullptr, stream2 = nullptr;
     // map
     SearchRow* rows = nullptr;
+    int corridor_levels = 0;  // corridor_levels() of the map: long corridors are searched by corridor.cu's kernel
+    EdgeRow* erow = nullptr;  // corridor maps: 4 per triangle
+    EdgeHalf* third = nullptr;  // corridor maps: per triangle
     float2* cen = nullptr;
     float2* tri = nullptr;
     int *gstart = nullptr, *glist = nullptr, *degen = nullptr;
@@ -262,11 +302,15 @@ struct Device {
     // search state
     Rec* rec = nullptr;
     unsigned* epoch = nullptr;
+    int4* log = nullptr;     // corridor maps: claim logs, slots x n
+    int* queues = nullptr;   // corridor maps: queues of the slots when they are not in shared memory
+    size_t queue_cap = 0;    // its bytes
+    int form = 0;            // SearchForm of the sized search
     int slots = 0;
     int vm = 2;                 // visited mode (1, 2 or 3; see launch_search)
     unsigned* gbm = nullptr;    // visited mode 3: slots x bm_words
     int bm_words = 0;           // bitmap words per slot
-    int rec_cap = 0, gbm_cap = 0;  // slots the record / bitmap arrays hold (kept across reshapes)
+    int rec_cap = 0, log_cap = 0, gbm_cap = 0;  // slots the records / logs / bitmaps hold (kept across reshapes)
     // agent grid
     int *cell_of = nullptr, *cell_cnt = nullptr, *cell_start = nullptr, *cell_fill = nullptr,
         *cell_items = nullptr;

@@ -631,6 +631,39 @@ __global__ void k_locate_points(LocateGrid g, const float2* pts, int n, int* out
     if (i < n) out[i] = locate(g, pts[i].x, pts[i].y);
 }
 
+// one thread per directed edge (v, s); see EdgeRow
+__global__ void k_edge_rows(const SearchRow* rows, int n, EdgeRow* out, EdgeHalf* third) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= 4ll * n) return;
+    const int v = (int)(k >> 2), s = (int)(k & 3);
+    const SearchRow r = rows[v];
+    const int nb[3] = {r.n0, r.n1, r.n2};
+    const float2 cen[3] = {make_float2(r.x0, r.y0), make_float2(r.x1, r.y1), make_float2(r.x2, r.y2)};
+    const int parent = s < r.deg ? nb[s] : -1;
+    EdgeRow o{{-1, (unsigned)r.deg << 4, 0.f, 0.f}, {-1, 0, 0.f, 0.f}};
+    EdgeHalf z{-1, 0, 0.f, 0.f};
+    int found = 0;
+    for (int j = 0; j < r.deg; j++) {
+        const int w = nb[j];
+        if (w == parent) continue;
+        const SearchRow& q = rows[w];
+        const int back = (q.deg > 0 && q.n0 == v) ? 0 : (q.deg > 1 && q.n1 == v) ? 1 : (q.deg > 2 && q.n2 == v) ? 2 : 3;
+        if (found < 2) {
+            EdgeHalf& h = found == 0 ? o.x : o.y;
+            h.e = w << 2 | back;
+            h.info |= 1u << j;
+            h.x = cen[j].x;
+            h.y = cen[j].y;
+        } else {
+            z = EdgeHalf{w << 2 | back, 4u, cen[j].x, cen[j].y};
+            o.x.info |= kEdgeThird;
+        }
+        found++;
+    }
+    out[k] = o;
+    if (s == 3) third[v] = z;  // (only a row that leaves no neighbour out has a third)
+}
+
 inline int blocks_for(int n, int bt) { return (n + bt - 1) / bt; }
 
 }  // namespace
@@ -665,6 +698,10 @@ void launch_prepare_batch(cudaStream_t s, const int* starts, const int* targets,
                           int4* req, int* req_count, int* work_ctr, int* err) {
     k_prepare_batch<<<blocks_for(n > 0 ? n : 1, 256), 256, 0, s>>>(starts, targets, n, nodes, req,
                                                                    req_count, work_ctr, err);
+}
+
+void launch_edge_rows(cudaStream_t s, const SearchRow* rows, int n, EdgeRow* out, EdgeHalf* third) {
+    k_edge_rows<<<(unsigned)((4ll * n + 255) / 256), 256, 0, s>>>(rows, n, out, third);
 }
 
 void launch_order_requests(cudaStream_t s, const int4* req_in, const int* req_count, int4* req_out, int* keys,

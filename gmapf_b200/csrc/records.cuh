@@ -1,4 +1,4 @@
-// records.cuh -- one 32-byte access per search record (device code only).
+// records.cuh -- search records and edge rows (device code only).
 //
 // A record (`Rec`, internal.h) is one 32-byte L2 sector.  Reading or writing
 // it with a single 256-bit access costs one L1 pass instead of two, and a
@@ -25,5 +25,30 @@ __device__ __forceinline__ void st_rec(Rec* r, unsigned stamp, int gd, int a0, i
                  "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(a4), "r"(a5)
                  : "memory");
 }
+
+// Lanes without a row (index < 0) issue no access: one shared dummy row would
+// make every warp of the GPU read the same sector in every round.
+__device__ __forceinline__ void ld_edge_half(const EdgeHalf* rows, long long k, EdgeHalf& o) {
+    asm volatile(
+        "{ .reg .pred p; setp.ge.s64 p, %5, 0; mov.b32 %0, -1; mov.b32 %1, 0; mov.f32 %2, 0f00000000; mov.f32 %3, 0f00000000;"
+        " @p ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4]; }"
+        : "=&r"(o.e), "=&r"(o.info), "=&f"(o.x), "=&f"(o.y)
+        : "l"(rows + k), "l"(k));
+}
+
+__device__ __forceinline__ void ld_edge_row(const EdgeRow* rows, int k, EdgeHalf& x, EdgeHalf& y) {
+    ld_edge_half(&rows->x, k < 0 ? -1 : 2 * (long long)k, x);
+    ld_edge_half(&rows->x, k < 0 ? -1 : 2 * (long long)k + 1, y);
+}
+
+// the row into shared memory, asynchronously; copies_done waits for this thread's copies
+__device__ __forceinline__ void copy_edge_row(EdgeHalf* to, const EdgeRow* rows, int k) {
+    if (k < 0) return;
+    const unsigned d = (unsigned)__cvta_generic_to_shared(to);
+    const EdgeRow* from = rows + k;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(&from->x) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16), "l"(&from->y) : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 }  // namespace gmapf_b200

@@ -149,6 +149,8 @@ struct Service {
     // the service's own search state
     Rec* rec = nullptr;
     unsigned* epoch = nullptr;
+    int4* log = nullptr;   // corridor maps, instead of rec
+    int* queues = nullptr;
     unsigned* gbm = nullptr;
     int slots = 0;
     unsigned long long* d_stats = nullptr;
@@ -235,6 +237,8 @@ SearchParams serve_params(Context& c, Service& sv, int k) {
     Device& d = c.dev;
     SearchParams p{};
     p.rows = d.rows;
+    p.erow = d.erow;
+    p.third = d.third;
     p.cen = d.cen;
     p.n = c.map.n;
     p.req = sv.d_ring;
@@ -245,6 +249,8 @@ SearchParams serve_params(Context& c, Service& sv, int k) {
     p.K = c.K;
     p.rec = sv.rec;
     p.epoch = sv.epoch;
+    p.log = sv.log;
+    p.queues = sv.queues;
     p.gbm = sv.gbm;
     p.slot_base = k * sv.slots_per_stream;
     p.slots = sv.slots_per_stream;
@@ -421,12 +427,12 @@ int serve_start(Context& c, int max_in_flight, std::string& err) {
     size_t freeb = 0, totalb = 0;
     SCK(cudaMemGetInfo(&freeb, &totalb));
     const int gpb = c.block_threads / 32;
-    const int per_sm = search_max_blocks_per_sm(c.T, c.C, c.block_threads, d.vm, d.bm_words);
+    const int per_sm = search_max_blocks_per_sm(c.T, c.C, c.block_threads, d.vm, d.bm_words, d.form);
     if (per_sm <= 0) {
         err = "serving: the search kernel cannot be resident with this shape";
         return GMAPF_E_CAPACITY;
     }
-    const double per_slot = (double)n * sizeof(Rec) + (d.vm >= 3 ? 4.0 * d.bm_words : 0.0);
+    const double per_slot = (double)search_slot_bytes(n, d.vm, d.bm_words, d.form);
     // the drain launch is persistent while queries keep coming: leave one
     // block per SM for the frames' own kernels
     const int drain_per_sm = per_sm > 1 ? per_sm - 1 : 1;
@@ -439,8 +445,13 @@ int serve_start(Context& c, int max_in_flight, std::string& err) {
     }
     sv.slots_per_stream = (int)per_stream;
     sv.slots = (int)(per_stream * kStreams);
-    SALLOC(sv.rec, (size_t)sv.slots * n);
-    SALLOC(sv.epoch, (size_t)sv.slots);
+    if (d.form == FORM_RECORDS) {
+        SALLOC(sv.rec, (size_t)sv.slots * n);
+        SALLOC(sv.epoch, (size_t)sv.slots);
+    } else {
+        SALLOC(sv.log, (size_t)sv.slots * n);
+        if (d.form == FORM_LOG_GLOBAL) SALLOC(sv.queues, sv.slots * corridor_queue_bytes(c.C, c.T) / sizeof(int));
+    }
     if (d.vm >= 3) SALLOC(sv.gbm, (size_t)sv.slots * d.bm_words);
     SALLOC(sv.d_stats, ST_COUNT);
 

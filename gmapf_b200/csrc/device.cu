@@ -218,6 +218,10 @@ MoverParams mover_params(Context& c) {
     return p;
 }
 
+OrderParams order_params(const Device& d, int2* keys) {
+    return OrderParams{d.lm, d.lm_count, d.lm_max, d.order_hist, keys};
+}
+
 CompactScenes compact_scenes(const Context& c) {
     const Device& d = c.dev;
     return CompactScenes{d.agent_scene, d.scene_abase, d.scene_P, d.scene_first};
@@ -405,14 +409,15 @@ int enqueue_frame(Context& c, bool timing, std::string& err) {
     if (timing) CK(cudaEventRecordWithFlags(d.ev[0], s, cudaEventRecordExternal));
     CK(cudaMemsetAsync(d.counters + CT_ERR, 0, sizeof(int), s));
     launch_compact(s, c.A, d.state, d.cur, d.targ, c.cfg.PathFinderParallelAgents, compact_scenes(c), d.req,
-                   d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_WORK, d.stats);
+                   d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_WORK, d.order_hist, d.stats);
     if (timing) CK(cudaEventRecordWithFlags(d.ev[1], s, cudaEventRecordExternal));
     CK(cudaEventRecord(d.ev[5], s));
     CK(cudaStreamWaitEvent(s2, d.ev[5], 0));
     // search branch (requests longest-first when the landmark estimate is on)
     SearchParams sp = search_params(c);
     if (d.lm) {
-        launch_order_requests(s, d.req, d.counters + CT_REQ, d.req_sorted, d.req_keys, d.lm, d.lm_count, c.map.n);
+        launch_order_requests(s, d.req, d.counters + CT_REQ, std::max(1, c.cfg.PathFinderParallelAgents), d.req_sorted,
+                              order_params(d, d.req_keys), c.map.n, d.slots);
         sp.req = d.req_sorted;
     }
     CK(launch_search(s, sp, search_blocks(c), c.block_threads, true, 0, d.vm, d.bm_words));
@@ -461,7 +466,8 @@ int capture_graph(Context& c, std::string& err) {
 }
 
 int kernels_per_frame(Context& c) {
-    return 2 + (c.dev.lm ? 1 : 0) + (c.A > 0 ? 4 + (c.dev.waypoints ? 1 : 0) : 0);
+    const bool sorted = c.dev.lm && std::max(1, c.cfg.PathFinderParallelAgents) > c.dev.slots;
+    return 2 + (c.dev.lm ? 1 : 0) + (sorted ? 1 : 0) + (c.A > 0 ? 4 + (c.dev.waypoints ? 1 : 0) : 0);
 }
 
 }  // namespace
@@ -550,6 +556,9 @@ int device_start(Context& c, std::string& err) {
         std::vector<unsigned short> lm;
         d.lm_count = 8;
         landmark_distances(m, d.lm_count, lm);
+        for (unsigned short v : lm)
+            if (v != 65535) d.lm_max = std::max<int>(d.lm_max, v);
+        DALLOC(d.order_hist, 1024);
         DALLOC(d.lm, lm.size());
         CK(cudaMemcpy(d.lm, lm.data(), sizeof(unsigned short) * lm.size(), cudaMemcpyHostToDevice));
         DALLOC(d.req_sorted, std::max(1, c.cfg.PathFinderParallelAgents));
@@ -701,7 +710,7 @@ int device_async_step(Context& c, float dt, std::string& err) {
         CK(cudaMemsetAsync(d.counters + CT_ERR, 0, sizeof(int), s));
         launch_compact(s, c.A, d.state, d.cur, d.targ, c.cfg.PathFinderParallelAgents, compact_scenes(c), d.req,
                        d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_WORK,
-                       d.stats);
+                       d.order_hist, d.stats);
         c.launches += 1;
         CK(cudaMemcpyAsync(c.h_small, d.counters, sizeof(int) * CT_COUNT, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -908,13 +917,14 @@ int device_search_batch(Context& c, const int* d_starts, const int* d_targets, i
     unsigned long long before[ST_COUNT];
     std::memcpy(before, c.h_stats, sizeof(before));
     launch_prepare_batch(s, d_starts, d_targets, n, c.map.n, d.breq, d.counters + CT_REQ,
-                         d.counters + CT_WORK, d.counters + CT_ERR);
+                         d.counters + CT_WORK, d.order_hist, d.counters + CT_ERR);
     c.launches += 1;
     SearchParams sp = search_params(c);
     sp.req = d.breq;
     if (d.lm && n > 0) {
-        launch_order_requests(s, d.breq, d.counters + CT_REQ, d.breq_sorted, d.breq_keys, d.lm, d.lm_count, c.map.n);
-        c.launches += 1;
+        launch_order_requests(s, d.breq, d.counters + CT_REQ, n, d.breq_sorted, order_params(d, d.breq_keys), c.map.n,
+                              d.slots);
+        c.launches += n > d.slots ? 2 : 1;
         sp.req = d.breq_sorted;
     }
     sp.paths = d_paths;

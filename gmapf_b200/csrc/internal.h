@@ -174,7 +174,7 @@ struct CompactScenes {
 };
 void launch_compact(cudaStream_t s, int A, int* state, const int* cur, const int* targ, int P,
                     const CompactScenes& scn, int4* req, int* req_count, unsigned char* in_move, int* mv_count,
-                    int* work_ctr, unsigned long long* stats);
+                    int* work_ctr, int* hist, unsigned long long* stats);
 void launch_apply_targets(cudaStream_t s, const int4* recs, int n, int* state, int* targ_node,
                           float2* targ_pos);
 // device-resident retargets of agents id_base + ids[k], ids[k] in [0, id_count)
@@ -183,9 +183,17 @@ void launch_locate_points(cudaStream_t s, const LocateGrid& g, const float2* pts
 void launch_apply_targets_device(cudaStream_t s, const int* ids, const float2* pos, int n, int id_base,
                                  int id_count, const ScenePar* sc, const int* agent_scene, int* state,
                                  int* targ_node, float2* targ_pos, int* err);
-// requests reordered longest-first by the landmark estimate (keys: scratch, one int per request)
-void launch_order_requests(cudaStream_t s, const int4* req_in, const int* req_count, int4* req_out, int* keys,
-                           const unsigned short* lm, int L, int n);
+// requests reordered longest-first by the landmark estimate (up to `most`
+// requests; with no more of them than slots they are only copied).  hist: 1,024
+// zeros (k_compact and k_prepare_batch clear it), keys: two ints per request
+struct OrderParams {
+    const unsigned short* lm;  // hop distances from L landmarks, L x n
+    int L, lm_max;             // lm_max: the largest of them (at least 1)
+    int* hist;
+    int2* keys;
+};
+void launch_order_requests(cudaStream_t s, const int4* req_in, const int* req_count, int most, int4* req_out,
+                           const OrderParams& o, int n, int slots);
 void launch_move_bin(cudaStream_t s, const MoverParams& p);
 void launch_cell_scan(cudaStream_t s, const MoverParams& p);
 void launch_scatter(cudaStream_t s, const MoverParams& p);
@@ -193,7 +201,7 @@ void launch_collide_progress(cudaStream_t s, const MoverParams& p);
 // path smoothing: funnel corners of the paths that start this frame
 void launch_funnel(cudaStream_t s, const MoverParams& p);
 void launch_prepare_batch(cudaStream_t s, const int* starts, const int* targets, int n, int nodes,
-                          int4* req, int* req_count, int* work_ctr, int* err);
+                          int4* req, int* req_count, int* work_ctr, int* hist, int* err);
 // the 4 n edge rows of a map with the given search rows
 void launch_edge_rows(cudaStream_t s, const SearchRow* rows, int n, EdgeRow* out, EdgeHalf* third);
 // search.cu
@@ -292,11 +300,12 @@ struct Device {
     // requests / counters
     int4* req = nullptr;
     int4* req_sorted = nullptr;  // longest-first order (order_by_estimate)
-    int* req_keys = nullptr;
+    int2* req_keys = nullptr;
     unsigned short* lm = nullptr;  // landmark hop distances, lm_count x n
-    int lm_count = 0;
+    int lm_count = 0, lm_max = 1;
+    int* order_hist = nullptr;
     int4* breq_sorted = nullptr;
-    int* breq_keys = nullptr;
+    int2* breq_keys = nullptr;
     int* counters = nullptr;  // [req_count, mv_count, work_ctr, err, spare...]
     unsigned long long* stats = nullptr;
     // search state

@@ -13,7 +13,10 @@
 // uniform grid whose cells are at least 1.0625 collision distances wide, so
 // the 3x3 neighbourhood holds every agent the reference's all-pairs loop
 // would accept.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "internal.h"
 
@@ -21,100 +24,163 @@ namespace gmapf_b200 {
 
 namespace {
 
-constexpr int kCompactThreads = 1024;
+namespace cg = cooperative_groups;
 
+constexpr int kOrderBuckets = 1024;  // of the longest-first order
+constexpr int kCompactThreads = 1024;
+constexpr int kCompactRun = 4;       // consecutive agents per thread and step
+constexpr int kCompactCluster = 8;   // thread blocks (one cluster) for more agents than one block's step
+
+// inclusive block scan (1,024 threads) of v; *total gets the sum.  warp_tot: 32 words
+__device__ __forceinline__ int block_scan(int v, int* warp_tot, int* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
+    }
+    __syncthreads();  // the previous scan's totals are read
+    if (lane == 31) warp_tot[warp] = v;
+    __syncthreads();
+    int w = warp_tot[lane];
+    for (int o = 1; o < 32; o <<= 1) {  // (every warp scans the 32 totals: no second barrier)
+        const int t = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += t;
+    }
+    *total = __shfl_sync(0xffffffffu, w, 31);
+    const int before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+    return v + (warp > 0 ? before : 0);
+}
+
+// block_scan over the cluster's blocks (CL of them) in rank order; cluster_tot:
+// CL words of shared memory, read by the other blocks
+template <int CL>
+__device__ __forceinline__ int cluster_scan(int v, int* warp_tot, int* cluster_tot, int* total) {
+    int tot;
+    const int incl = block_scan(v, warp_tot, &tot);
+    if constexpr (CL == 1) {
+        *total = tot;
+        return incl;
+    } else {
+        cg::cluster_group cl = cg::this_cluster();
+        cl.sync();  // the previous scan's totals are read
+        if (threadIdx.x < CL) cl.map_shared_rank(cluster_tot, threadIdx.x)[cl.block_rank()] = tot;
+        cl.sync();
+        int before = 0, all = 0;
+#pragma unroll
+        for (int k = 0; k < CL; k++) {
+            const int t = cluster_tot[k];
+            before += k < (int)cl.block_rank() ? t : 0;
+            all += t;
+        }
+        *total = all;
+        return before + incl;
+    }
+}
+
+// Request compaction: four agents per thread and step, one scan of both counts
+// (Search agents in the low half, Move agents in the high half: at most 32,768
+// of each per step).  It reads and writes 10 to 40 bytes per agent and is bound
+// by latency: loads, scan, stores, one after the other.  One block of 4,096
+// agents a step up to that many, beyond it a cluster of eight blocks whose
+// totals go through distributed shared memory, 32,768 agents a step: 7.9 us for
+// 16,384 requests and 10.4 us for 24,000 agents in 64 scenes.  (One block with
+// one agent per thread and three barriers per scan took 29 and 63 us; the same
+// block with 16 agents per thread 34 and 23 us.)
+//
 // Per-scene request limits (a scene batch): scene s takes its Search agents in
 // ascending id up to P[s] (each scene is its own PathFinder, PathFinder.h:76-117).
 // first[s] records how many Search agents precede the scene's first agent.
-__global__ void __launch_bounds__(kCompactThreads)
-    k_compact(int A, int* state, const int* cur, const int* targ, int P, CompactScenes scn, int4* req,
-              int* req_count, unsigned char* in_move, int* mv_count, int* work_ctr, unsigned long long* stats) {
+template <int CL>
+__device__ __forceinline__ void compact(int A, int* state, const int* cur, const int* targ, int P, const CompactScenes& scn,
+                                        int4* req, int* req_count, unsigned char* in_move, int* mv_count, int* work_ctr,
+                                        int* hist, unsigned long long* stats) {
     __shared__ int warp_tot[32];
-    __shared__ int warp_totm[32];
-    __shared__ int warp_toto[32];
-    __shared__ int base_s, base_m, base_o;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const unsigned lt = (1u << lane) - 1u;
+    __shared__ int cluster_tot[CL];
+    const int tid = threadIdx.x;
+    const int rank = CL > 1 ? (int)blockIdx.x : 0;
     const bool scenes = scn.agent_scene != nullptr;
-    if (tid == 0) {
-        base_s = 0;
-        base_m = 0;
-        base_o = 0;
-    }
-    __syncthreads();
-    for (int b = 0; b < A; b += kCompactThreads) {
-        const int i = b + tid;
-        bool isS = false, isM = false;
-        int cu = 0, ta = 0;
-        if (i < A) {
-            const int st = state[i];
-            if (st == GMAPF_AGENT_SEARCH) {
-                cu = cur[i];
-                ta = targ[i];
-                if (cu == ta) {
-                    state[i] = GMAPF_AGENT_IDLE;  // PathFinder.h:91-95
-                } else {
-                    isS = true;
-                }
-            }
-            isM = st == GMAPF_AGENT_MOVE;
-            in_move[i] = isM ? 1 : 0;
-        }
-        const unsigned bs = __ballot_sync(0xffffffffu, isS);
-        const unsigned bm = __ballot_sync(0xffffffffu, isM);
-        if (lane == 0) {
-            warp_tot[warp] = __popc(bs);
-            warp_totm[warp] = __popc(bm);
-        }
-        __syncthreads();
-        if (warp == 0) {
-            int v = warp_tot[lane], vm = warp_totm[lane];
-            // inclusive scans over the 32 warp totals
-            for (int o = 1; o < 32; o <<= 1) {
-                int t = __shfl_up_sync(0xffffffffu, v, o);
-                int tm = __shfl_up_sync(0xffffffffu, vm, o);
-                if (lane >= o) {
-                    v += t;
-                    vm += tm;
-                }
-            }
-            warp_tot[lane] = v;  // inclusive
-            warp_totm[lane] = vm;
-        }
-        __syncthreads();
-        const int wpre = (warp == 0) ? 0 : warp_tot[warp - 1];
-        const int gpos = base_s + wpre + __popc(bs & lt);  // Search agents before i
-        if (!scenes) {
-            if (isS && gpos < P) req[gpos] = make_int4(i, cu, ta, i);  // over capacity: stays Search
+    static_assert(kOrderBuckets == kCompactThreads, "one bucket per thread");
+    if (hist && rank == 0) hist[tid] = 0;  // the order's buckets
+    int base_s = 0, base_m = 0, base_o = 0;  // before this step (the same on every thread)
+    for (int b = 0; b < A; b += CL * kCompactThreads * kCompactRun) {
+        const int i0 = b + (rank * kCompactThreads + tid) * kCompactRun;
+        const int cnt = max(0, min(kCompactRun, A - i0));
+        int st[kCompactRun], cu[kCompactRun], ta[kCompactRun];
+        if (cnt == kCompactRun) {  // (runs of 4 start on 16-byte boundaries)
+            auto load = [&](const int* from, int* to) {
+                const int4 q = *reinterpret_cast<const int4*>(from + i0);
+                to[0] = q.x;
+                to[1] = q.y;
+                to[2] = q.z;
+                to[3] = q.w;
+            };
+            load(state, st);
+            load(cur, cu);
+            load(targ, ta);
         } else {
-            const int sidx = i < A ? scn.agent_scene[i] : 0;
-            if (i < A && i == scn.abase[sidx]) scn.first[sidx] = gpos;
-            __syncthreads();
-            const bool ok = isS && gpos - scn.first[sidx] < scn.P[sidx];
-            const unsigned bo = __ballot_sync(0xffffffffu, ok);
-            if (lane == 0) warp_toto[warp] = __popc(bo);
-            __syncthreads();
-            if (warp == 0) {
-                int v = warp_toto[lane];
-                for (int o = 1; o < 32; o <<= 1) {
-                    int t = __shfl_up_sync(0xffffffffu, v, o);
-                    if (lane >= o) v += t;
-                }
-                warp_toto[lane] = v;
+#pragma unroll
+            for (int j = 0; j < kCompactRun; j++) {
+                st[j] = j < cnt ? state[i0 + j] : GMAPF_AGENT_IDLE;
+                cu[j] = j < cnt ? cur[i0 + j] : 0;
+                ta[j] = j < cnt ? targ[i0 + j] : 0;
             }
-            __syncthreads();
-            const int opos = base_o + (warp == 0 ? 0 : warp_toto[warp - 1]) + __popc(bo & lt);
-            if (ok) req[opos] = make_int4(i, cu, ta, i);
         }
-        __syncthreads();
-        if (tid == 0) {
-            base_s += warp_tot[31];
-            base_m += warp_totm[31];
-            if (scenes) base_o += warp_toto[31];
+        bool want[kCompactRun];
+        int ns = 0, nm = 0;
+        unsigned flags = 0;
+#pragma unroll
+        for (int j = 0; j < kCompactRun; j++) {
+            want[j] = st[j] == GMAPF_AGENT_SEARCH && cu[j] != ta[j];
+            if (st[j] == GMAPF_AGENT_SEARCH && !want[j]) state[i0 + j] = GMAPF_AGENT_IDLE;  // PathFinder.h:91-95
+            const bool m = st[j] == GMAPF_AGENT_MOVE;
+            ns += want[j];
+            nm += m;
+            flags |= (m ? 1u : 0u) << (8 * j);
         }
-        __syncthreads();
+        if (cnt == kCompactRun)
+            *reinterpret_cast<unsigned*>(in_move + i0) = flags;
+        else
+            for (int j = 0; j < cnt; j++) in_move[i0 + j] = (flags >> (8 * j)) & 1u;
+        int tot;
+        const int incl = cluster_scan<CL>(ns | nm << 16, warp_tot, cluster_tot, &tot);
+        int pos = base_s + (incl & 0xffff) - ns;  // Search agents before this run
+        if (!scenes) {
+#pragma unroll
+            for (int j = 0; j < kCompactRun; j++)
+                if (want[j]) {
+                    if (pos < P) req[pos] = make_int4(i0 + j, cu[j], ta[j], i0 + j);  // over capacity: stays Search
+                    pos++;
+                }
+        } else {
+            int sidx[kCompactRun], at[kCompactRun];
+#pragma unroll
+            for (int j = 0; j < kCompactRun; j++) {
+                sidx[j] = j < cnt ? scn.agent_scene[i0 + j] : 0;
+                at[j] = pos;
+                if (j < cnt && i0 + j == scn.abase[sidx[j]]) scn.first[sidx[j]] = pos;
+                pos += want[j];
+            }
+            if constexpr (CL == 1)
+                __syncthreads();
+            else
+                cg::this_cluster().sync();
+            int ok = 0;
+#pragma unroll
+            for (int j = 0; j < kCompactRun; j++) {
+                want[j] = want[j] && at[j] - __ldcg(scn.first + sidx[j]) < scn.P[sidx[j]];
+                ok += want[j];
+            }
+            int tot_o;
+            int opos = base_o + cluster_scan<CL>(ok, warp_tot, cluster_tot, &tot_o) - ok;
+#pragma unroll
+            for (int j = 0; j < kCompactRun; j++)
+                if (want[j]) req[opos++] = make_int4(i0 + j, cu[j], ta[j], i0 + j);
+            base_o += tot_o;
+        }
+        base_s += tot & 0xffff;
+        base_m += (int)((unsigned)tot >> 16);
     }
-    if (tid == 0) {
+    if (tid == 0 && rank == 0) {
         const int R = scenes ? base_o : (base_s < P ? base_s : P);
         *req_count = R;
         *mv_count = base_m;
@@ -122,7 +188,20 @@ __global__ void __launch_bounds__(kCompactThreads)
         stats[ST_REQUESTS] += (unsigned long long)R;
         stats[ST_MOVING] += (unsigned long long)base_m;
     }
+    if constexpr (CL > 1) cg::this_cluster().sync();  // no block leaves while another may still write its totals
 }
+
+#define COMPACT_ARGS                                                                                          \
+    int A, int *state, const int *cur, const int *targ, int P, CompactScenes scn, int4 *req, int *req_count, \
+        unsigned char *in_move, int *mv_count, int *work_ctr, int *hist, unsigned long long *stats
+__global__ void __launch_bounds__(kCompactThreads) k_compact(COMPACT_ARGS) {
+    compact<1>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, work_ctr, hist, stats);
+}
+__global__ void __cluster_dims__(kCompactCluster, 1, 1) __launch_bounds__(kCompactThreads)
+    k_compact_cluster(COMPACT_ARGS) {
+    compact<kCompactCluster>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, work_ctr, hist, stats);
+}
+#undef COMPACT_ARGS
 
 __global__ void k_apply_targets(const int4* recs, int n, int* state, int* targ_node,
                                 float2* targ_pos) {
@@ -159,8 +238,10 @@ __global__ void k_apply_targets_device(const int* ids, const float2* pos, int n,
 }
 
 __global__ void k_prepare_batch(const int* starts, const int* targets, int n, int nodes, int4* req,
-                                int* req_count, int* work_ctr, int* err) {
+                                int* req_count, int* work_ctr, int* hist, int* err) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (hist && blockIdx.x == 0)  // the order's buckets
+        for (int j = threadIdx.x; j < kOrderBuckets; j += blockDim.x) hist[j] = 0;
     if (k == 0) {
         *req_count = n;
         *work_ctr = 0;
@@ -175,70 +256,50 @@ __global__ void k_prepare_batch(const int* starts, const int* targets, int n, in
 // the landmark lower bound on the hop distance, max_l |d_l(s) - d_l(t)|, and
 // requests are bucketed by it in descending order.  Results do not depend
 // on the order (every request writes only its own row and agent).
-constexpr int kOrderBuckets = 1024;
-
-__global__ void __launch_bounds__(1024) k_order_requests(const int4* req_in, const int* req_count, int4* req_out,
-                                                         int* keys, const unsigned short* lm, int L, int n) {
-    __shared__ int hist[kOrderBuckets];
-    __shared__ int wmax[32];
-    __shared__ int gmax;
-    const int tid = threadIdx.x;
+//
+// Two launches over all SMs (16 scattered 2-byte reads per request, then one
+// read and one write of it): one block for all requests took 80 us at 16,384
+// requests and 11.5 us at 2,048, now 8.6 + 4.7 and 2.7.  The buckets are scaled by the
+// map's largest landmark distance, so that no pass over the estimates has to
+// find their maximum first.  With a search slot for every request the order is
+// of no use: they are copied.
+__global__ void __launch_bounds__(256) k_order_keys(const int4* req_in, const int* req_count, int4* req_out, int2* keys,
+                                                    int* hist, const unsigned short* lm, int L, int n, int lm_max,
+                                                    int slots) {
     const int R = *req_count;
-    int mx = 0;
-    for (int i = tid; i < R; i += blockDim.x) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < R; i += gridDim.x * blockDim.x) {
         const int4 q = req_in[i];
+        if (R <= slots) {
+            req_out[i] = q;
+            continue;
+        }
         int est = 0;
         if (q.y >= 0 && q.y < n && q.z >= 0 && q.z < n) {
+#pragma unroll 8
             for (int l = 0; l < L; l++) {
                 const int a = lm[(size_t)l * n + q.y], b = lm[(size_t)l * n + q.z];
                 const int e = (a == 65535 || b == 65535) ? 65535 : abs(a - b);
                 est = max(est, e);
             }
         }
-        keys[i] = est;
-        mx = max(mx, est);
+        const int b = (kOrderBuckets - 1) - (int)((long long)min(est, lm_max) * (kOrderBuckets - 1) / lm_max);
+        keys[i] = make_int2(b, atomicAdd(hist + b, 1));
     }
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((tid & 31) == 0) wmax[tid >> 5] = mx;
-    hist[tid] = 0;
+}
+
+__global__ void __launch_bounds__(1024) k_order_place(const int4* req_in, const int* req_count, int4* req_out,
+                                                      const int2* keys, const int* hist, int slots) {
+    __shared__ int warp_tot[32];
+    __shared__ int start[kOrderBuckets];
+    const int R = *req_count;
+    if (R <= slots) return;
+    const int h = hist[threadIdx.x];
+    int tot;
+    start[threadIdx.x] = block_scan(h, warp_tot, &tot) - h;
     __syncthreads();
-    if (tid < 32) {
-        int v = wmax[tid];
-        for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (tid == 0) gmax = v;
-    }
-    __syncthreads();
-    const long long den = max(1, gmax);
-    for (int i = tid; i < R; i += blockDim.x) {
-        const int b = (kOrderBuckets - 1) - (int)(((long long)keys[i] * (kOrderBuckets - 1)) / den);
-        keys[i] = b;
-        atomicAdd(hist + b, 1);
-    }
-    __syncthreads();
-    // exclusive scan of the histogram (one value per thread)
-    int v = hist[tid];
-    const int lane = tid & 31, w = tid >> 5;
-    int x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) wmax[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        int s = wmax[lane];
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += y;
-        }
-        wmax[lane] = s;  // inclusive warp sums
-    }
-    __syncthreads();
-    hist[tid] = x - v + (w > 0 ? wmax[w - 1] : 0);
-    __syncthreads();
-    for (int i = tid; i < R; i += blockDim.x) {
-        const int pos = atomicAdd(hist + keys[i], 1);
-        req_out[pos] = req_in[i];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < R; i += gridDim.x * blockDim.x) {
+        const int2 k = keys[i];
+        req_out[start[k.x] + k.y] = req_in[i];
     }
 }
 
@@ -670,9 +731,13 @@ inline int blocks_for(int n, int bt) { return (n + bt - 1) / bt; }
 
 void launch_compact(cudaStream_t s, int A, int* state, const int* cur, const int* targ, int P,
                     const CompactScenes& scn, int4* req, int* req_count, unsigned char* in_move, int* mv_count,
-                    int* work_ctr, unsigned long long* stats) {
-    k_compact<<<1, kCompactThreads, 0, s>>>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count,
-                                            work_ctr, stats);
+                    int* work_ctr, int* hist, unsigned long long* stats) {
+    if (A <= kCompactThreads * kCompactRun)
+        k_compact<<<1, kCompactThreads, 0, s>>>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count,
+                                                work_ctr, hist, stats);
+    else
+        k_compact_cluster<<<kCompactCluster, kCompactThreads, 0, s>>>(A, state, cur, targ, P, scn, req, req_count,
+                                                                      in_move, mv_count, work_ctr, hist, stats);
 }
 
 void launch_apply_targets(cudaStream_t s, const int4* recs, int n, int* state, int* targ_node,
@@ -695,18 +760,22 @@ void launch_apply_targets_device(cudaStream_t s, const int* ids, const float2* p
 }
 
 void launch_prepare_batch(cudaStream_t s, const int* starts, const int* targets, int n, int nodes,
-                          int4* req, int* req_count, int* work_ctr, int* err) {
+                          int4* req, int* req_count, int* work_ctr, int* hist, int* err) {
     k_prepare_batch<<<blocks_for(n > 0 ? n : 1, 256), 256, 0, s>>>(starts, targets, n, nodes, req,
-                                                                   req_count, work_ctr, err);
+                                                                   req_count, work_ctr, hist, err);
 }
 
 void launch_edge_rows(cudaStream_t s, const SearchRow* rows, int n, EdgeRow* out, EdgeHalf* third) {
     k_edge_rows<<<(unsigned)((4ll * n + 255) / 256), 256, 0, s>>>(rows, n, out, third);
 }
 
-void launch_order_requests(cudaStream_t s, const int4* req_in, const int* req_count, int4* req_out, int* keys,
-                           const unsigned short* lm, int L, int n) {
-    k_order_requests<<<1, 1024, 0, s>>>(req_in, req_count, req_out, keys, lm, L, n);
+void launch_order_requests(cudaStream_t s, const int4* req_in, const int* req_count, int most, int4* req_out,
+                           const OrderParams& o, int n, int slots) {
+    const int blocks = std::max(1, std::min(128, blocks_for(most, 256)));
+    k_order_keys<<<blocks, 256, 0, s>>>(req_in, req_count, req_out, o.keys, o.hist, o.lm, o.L, n, o.lm_max, slots);
+    if (most > slots)
+        k_order_place<<<std::min(32, blocks_for(most, 1024)), 1024, 0, s>>>(req_in, req_count, req_out, o.keys, o.hist,
+                                                                           slots);
 }
 
 void launch_move_bin(cudaStream_t s, const MoverParams& p) {

@@ -54,7 +54,7 @@ int search_promote_rounds(const Context& c) { return c.opt.promote_rounds > 0 ? 
 namespace {
 
 // device counters: [8] holds the frame's dt as a float
-enum Counter { CT_REQ = 0, CT_MOVE = 1, CT_WORK = 2, CT_ERR = 3, CT_ERR_TARGETS = 4, CT_COUNT = 16 };
+enum Counter { CT_REQ = 0, CT_MOVE = 1, CT_WORK = 2, CT_ERR = 3, CT_ERR_TARGETS = 4, CT_PARITY = 9, CT_COUNT = 16 };
 
 template <class T>
 int dalloc(Context& c, T** p, size_t count, std::string& err) {
@@ -205,10 +205,10 @@ MoverParams mover_params(Context& c) {
     p.agent_scene = d.agent_scene;
     p.cells = d.cells;
     p.cell_of = d.cell_of;
-    p.cell_cnt = d.cell_cnt;
-    p.cell_start = d.cell_start;
-    p.cell_fill = d.cell_fill;
-    p.cell_items = d.cell_items;
+    p.parity = d.counters + CT_PARITY;
+    p.cell_head = d.cell_head;
+    p.bucket = d.bucket;
+    p.next = d.next;
     p.tri = d.tri;
     p.cen = d.cen;
     p.waypoints = d.waypoints;
@@ -409,7 +409,8 @@ int enqueue_frame(Context& c, bool timing, std::string& err) {
     if (timing) CK(cudaEventRecordWithFlags(d.ev[0], s, cudaEventRecordExternal));
     CK(cudaMemsetAsync(d.counters + CT_ERR, 0, sizeof(int), s));
     launch_compact(s, c.A, d.state, d.cur, d.targ, c.cfg.PathFinderParallelAgents, compact_scenes(c), d.req,
-                   d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_WORK, d.order_hist, d.stats);
+                   d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_PARITY,
+                   d.counters + CT_WORK, d.order_hist, d.stats);
     if (timing) CK(cudaEventRecordWithFlags(d.ev[1], s, cudaEventRecordExternal));
     CK(cudaEventRecord(d.ev[5], s));
     CK(cudaStreamWaitEvent(s2, d.ev[5], 0));
@@ -425,11 +426,8 @@ int enqueue_frame(Context& c, bool timing, std::string& err) {
     // mover branch
     MoverParams mp = mover_params(c);
     if (c.A > 0) {
-        CK(cudaMemsetAsync(d.cell_cnt, 0, sizeof(int) * (d.cells + 1), s2));
         launch_funnel(s2, mp);  // path smoothing only
         launch_move_bin(s2, mp);
-        launch_cell_scan(s2, mp);
-        launch_scatter(s2, mp);
         launch_collide_progress(s2, mp);
     }
     if (timing) CK(cudaEventRecordWithFlags(d.ev[3], s2, cudaEventRecordExternal));
@@ -467,7 +465,7 @@ int capture_graph(Context& c, std::string& err) {
 
 int kernels_per_frame(Context& c) {
     const bool sorted = c.dev.lm && std::max(1, c.cfg.PathFinderParallelAgents) > c.dev.slots;
-    return 2 + (c.dev.lm ? 1 : 0) + (sorted ? 1 : 0) + (c.A > 0 ? 4 + (c.dev.waypoints ? 1 : 0) : 0);
+    return 2 + (c.dev.lm ? 1 : 0) + (sorted ? 1 : 0) + (c.A > 0 ? 2 + (c.dev.waypoints ? 1 : 0) : 0);
 }
 
 }  // namespace
@@ -606,10 +604,9 @@ int device_start(Context& c, std::string& err) {
         CK(cudaMemcpy(d.scene_P, sp.data(), sizeof(int) * sp.size(), cudaMemcpyHostToDevice));
     }
     DALLOC(d.cell_of, A);
-    DALLOC(d.cell_cnt, (size_t)d.cells + 1);
-    DALLOC(d.cell_start, (size_t)d.cells + 1);
-    DALLOC(d.cell_fill, (size_t)d.cells + 1);
-    DALLOC(d.cell_items, A);
+    DALLOC(d.cell_head, 2 * (size_t)d.cells);
+    DALLOC(d.bucket, 4 * (size_t)d.cells);
+    DALLOC(d.next, A);
 
     // pinned host staging
     CK(cudaMallocHost((void**)&c.h_pos_stage, sizeof(float2) * std::max(1, A)));
@@ -709,8 +706,8 @@ int device_async_step(Context& c, float dt, std::string& err) {
         if (timing) CK(cudaEventRecord(d.ev[0], s));
         CK(cudaMemsetAsync(d.counters + CT_ERR, 0, sizeof(int), s));
         launch_compact(s, c.A, d.state, d.cur, d.targ, c.cfg.PathFinderParallelAgents, compact_scenes(c), d.req,
-                       d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_WORK,
-                       d.order_hist, d.stats);
+                       d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_PARITY,
+                       d.counters + CT_WORK, d.order_hist, d.stats);
         c.launches += 1;
         CK(cudaMemcpyAsync(c.h_small, d.counters, sizeof(int) * CT_COUNT, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -733,13 +730,10 @@ int device_async_step(Context& c, float dt, std::string& err) {
         if (timing) CK(cudaEventRecord(d.ev[2], s));
         if (M > 0) {
             MoverParams mp = mover_params(c);
-            CK(cudaMemsetAsync(d.cell_cnt, 0, sizeof(int) * (d.cells + 1), s));
             launch_funnel(s, mp);  // path smoothing only
             launch_move_bin(s, mp);
-            launch_cell_scan(s, mp);
-            launch_scatter(s, mp);
             launch_collide_progress(s, mp);
-            c.launches += 4 + (d.waypoints ? 1 : 0);
+            c.launches += 2 + (d.waypoints ? 1 : 0);
         }
         if (timing) CK(cudaEventRecord(d.ev[3], s));
         if (c.A > 0) {

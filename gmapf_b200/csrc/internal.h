@@ -149,10 +149,10 @@ struct MoverParams {
     // agent grid (all scenes' cells, global ids)
     int cells;
     int* cell_of;
-    int* cell_cnt;     // cells + 1
-    int* cell_start;   // cells + 1
-    int* cell_fill;    // cells
-    int* cell_items;   // A
+    const int* parity; // whose turn of the two copies of cell_head it is
+    int2* cell_head;   // 2 x cells: agents in the cell, list of those beyond its bucket
+    int* bucket;       // 4 x cells: the first agents of a cell
+    int* next;         // A: the lists
     // map
     const float2* tri; // 3 vertices per triangle, global ids
     const float2* cen;
@@ -174,7 +174,7 @@ struct CompactScenes {
 };
 void launch_compact(cudaStream_t s, int A, int* state, const int* cur, const int* targ, int P,
                     const CompactScenes& scn, int4* req, int* req_count, unsigned char* in_move, int* mv_count,
-                    int* work_ctr, int* hist, unsigned long long* stats);
+                    int* parity, int* work_ctr, int* hist, unsigned long long* stats);
 void launch_apply_targets(cudaStream_t s, const int4* recs, int n, int* state, int* targ_node,
                           float2* targ_pos);
 // device-resident retargets of agents id_base + ids[k], ids[k] in [0, id_count)
@@ -195,8 +195,6 @@ struct OrderParams {
 void launch_order_requests(cudaStream_t s, const int4* req_in, const int* req_count, int most, int4* req_out,
                            const OrderParams& o, int n, int slots);
 void launch_move_bin(cudaStream_t s, const MoverParams& p);
-void launch_cell_scan(cudaStream_t s, const MoverParams& p);
-void launch_scatter(cudaStream_t s, const MoverParams& p);
 void launch_collide_progress(cudaStream_t s, const MoverParams& p);
 // path smoothing: funnel corners of the paths that start this frame
 void launch_funnel(cudaStream_t s, const MoverParams& p);
@@ -321,8 +319,8 @@ struct Device {
     int bm_words = 0;           // bitmap words per slot
     int rec_cap = 0, log_cap = 0, gbm_cap = 0;  // slots the records / logs / bitmaps hold (kept across reshapes)
     // agent grid
-    int *cell_of = nullptr, *cell_cnt = nullptr, *cell_start = nullptr, *cell_fill = nullptr,
-        *cell_items = nullptr;
+    int *cell_of = nullptr, *bucket = nullptr, *next = nullptr;
+    int2* cell_head = nullptr;
     int cells = 0;
     // scenes (ScenePar per scene; the rest only when there is more than one)
     ScenePar* scene_par = nullptr;

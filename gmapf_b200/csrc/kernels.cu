@@ -9,8 +9,8 @@
 // Agents are stored as structure-of-arrays.  Compaction is stable (requests
 // in ascending agent id).  Collisions read one snapshot of the positions
 // after the move and write a second buffer (Jacobi); each agent sums its
-// contributions in ascending neighbour id, found through a counting-sort
-// uniform grid whose cells are at least 1.0625 collision distances wide, so
+// contributions in ascending neighbour id, found through a uniform grid whose
+// cells are at least 1.0625 collision distances wide, so
 // the 3x3 neighbourhood holds every agent the reference's all-pairs loop
 // would accept.
 #include <cooperative_groups.h>
@@ -92,8 +92,8 @@ __device__ __forceinline__ int cluster_scan(int v, int* warp_tot, int* cluster_t
 // first[s] records how many Search agents precede the scene's first agent.
 template <int CL>
 __device__ __forceinline__ void compact(int A, int* state, const int* cur, const int* targ, int P, const CompactScenes& scn,
-                                        int4* req, int* req_count, unsigned char* in_move, int* mv_count, int* work_ctr,
-                                        int* hist, unsigned long long* stats) {
+                                        int4* req, int* req_count, unsigned char* in_move, int* mv_count, int* parity,
+                                        int* work_ctr, int* hist, unsigned long long* stats) {
     __shared__ int warp_tot[32];
     __shared__ int cluster_tot[CL];
     const int tid = threadIdx.x;
@@ -184,6 +184,7 @@ __device__ __forceinline__ void compact(int A, int* state, const int* cur, const
         const int R = scenes ? base_o : (base_s < P ? base_s : P);
         *req_count = R;
         *mv_count = base_m;
+        if (base_m > 0) *parity ^= 1;  // the mover runs: its grid takes turns
         *work_ctr = 0;
         stats[ST_REQUESTS] += (unsigned long long)R;
         stats[ST_MOVING] += (unsigned long long)base_m;
@@ -193,13 +194,13 @@ __device__ __forceinline__ void compact(int A, int* state, const int* cur, const
 
 #define COMPACT_ARGS                                                                                          \
     int A, int *state, const int *cur, const int *targ, int P, CompactScenes scn, int4 *req, int *req_count, \
-        unsigned char *in_move, int *mv_count, int *work_ctr, int *hist, unsigned long long *stats
+        unsigned char *in_move, int *mv_count, int *parity, int *work_ctr, int *hist, unsigned long long *stats
 __global__ void __launch_bounds__(kCompactThreads) k_compact(COMPACT_ARGS) {
-    compact<1>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, work_ctr, hist, stats);
+    compact<1>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, parity, work_ctr, hist, stats);
 }
 __global__ void __cluster_dims__(kCompactCluster, 1, 1) __launch_bounds__(kCompactThreads)
     k_compact_cluster(COMPACT_ARGS) {
-    compact<kCompactCluster>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, work_ctr, hist, stats);
+    compact<kCompactCluster>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, parity, work_ctr, hist, stats);
 }
 #undef COMPACT_ARGS
 
@@ -303,10 +304,23 @@ __global__ void __launch_bounds__(1024) k_order_place(const int4* req_in, const 
     }
 }
 
-// move (AgentsMover.h:51-71) fused with the agent-grid histogram
+// The agent grid of a frame: per cell a count and, for the agents beyond the
+// four of its bucket, the head of a list (agent + 1, 0: none).  Cells hold about
+// one agent on average (5% of the agents of a uniform crowd find their bucket
+// full), so one 16-byte read gives a cell's agents, and binning is one pass: no
+// scan over the cells and no second pass to place the agents (k_cell_scan and
+// k_scatter took 4 + 4 us at 2,048 agents, 39 + 4 us at 24,000 in 64 scenes).
+// Two copies of the counts take turns, so that a frame's binning clears the
+// other frame's without a launch of its own; *p.parity says whose turn it is.
+constexpr int kBucket = 4;
+
+// move (AgentsMover.h:51-71) fused with the binning
 __global__ void k_move_bin(MoverParams p) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (*p.mv_count == 0) return;  // AgentsMover.h:296-297
+    const int turn = *p.parity & 1;
+    int2* const old = p.cell_head + (size_t)(1 - turn) * p.cells;
+    for (int k = i; k < p.cells; k += gridDim.x * blockDim.x) old[k] = make_int2(0, 0);
     if (i >= p.A) return;
     const ScenePar& sc = p.sc[p.agent_scene ? p.agent_scene[i] : 0];
     float2 c = p.pos[i];
@@ -328,143 +342,161 @@ __global__ void k_move_bin(MoverParams p) {
         const int cx = grid_cell(c.x, sc.ax0, sc.ainv, sc.aw);
         const int cy = grid_cell(c.y, sc.ay0, sc.ainv, sc.ah);
         cell = sc.cell_base + cy * sc.aw + cx;
-        atomicAdd(p.cell_cnt + cell, 1);
+        int2* const h = p.cell_head + (size_t)turn * p.cells + cell;
+        const int k = atomicAdd(&h->x, 1);
+        if (k < kBucket)
+            p.bucket[kBucket * (size_t)cell + k] = i;
+        else
+            p.next[i] = atomicExch(&h->y, i + 1);
     }
     p.cell_of[i] = cell;
 }
 
-// exclusive scan of the cell histogram, one block: each thread sums a run of
-// cells, the runs are scanned with warp shuffles (two block barriers), then
-// each thread writes its run's starts
-__global__ void __launch_bounds__(1024) k_cell_scan(MoverParams p) {
-    if (*p.mv_count == 0) return;
-    __shared__ int wsum[32];
-    const int cells = p.cells;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int per = (cells + 1023) / 1024;
-    const int b = tid * per, e = min(b + per, cells);
-    int s = 0;
-#pragma unroll 8
-    for (int k = b; k < e; k++) s += p.cell_cnt[k];  // unrolled: the loads of a run are in flight together
-    int x = s;  // inclusive scan of the runs within the warp
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        int v = wsum[lane];
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += y;
-        }
-        wsum[lane] = v;  // inclusive warp totals
-    }
-    __syncthreads();
-    int run = x - s + (w > 0 ? wsum[w - 1] : 0);
-#pragma unroll 8
-    for (int k = b; k < e; k++) {
-        p.cell_start[k] = run;
-        p.cell_fill[k] = run;
-        run += p.cell_cnt[k];
-    }
-    if (tid == 1023) p.cell_start[cells] = wsum[31];
-}
-
-__global__ void k_scatter(MoverParams p) {
-    if (*p.mv_count == 0) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.A) return;
-    const int c = p.cell_of[i];
-    if (c < 0) return;
-    const int k = atomicAdd(p.cell_fill + c, 1);
-    p.cell_items[k] = i;
-}
-
 constexpr int kMaxLocal = 16;
 
+// The agents pushing one agent, with their contributions, ids ascending
+struct Pushes {
+    int ids[kMaxLocal];
+    float vx[kMaxLocal], vy[kMaxLocal];
+    int cnt = 0;
+    bool overflow = false;
+    __device__ __forceinline__ void add(int j, float dx, float dy, float d2, float cd) {
+        if (cnt >= kMaxLocal) {
+            overflow = true;
+            return;
+        }
+        const float d = GM_FSQRT(d2);
+        const float shift = GM_FSUB(cd, d);
+        const float x = GM_FMUL(GM_FDIV(dx, d), shift);
+        const float y = GM_FMUL(GM_FDIV(dy, d), shift);
+        int k = cnt++;
+        while (k > 0 && ids[k - 1] > j) {
+            ids[k] = ids[k - 1];
+            vx[k] = vx[k - 1];
+            vy[k] = vy[k - 1];
+            k--;
+        }
+        ids[k] = j;
+        vx[k] = x;
+        vy[k] = y;
+    }
+};
+
 // collisions (AgentsMover.h:73-129) + path progress (AgentsMover.h:131-177)
-__global__ void k_collide_progress(MoverParams p) {
+//
+// One agent per thread, bound by its chain of dependent reads, not by their
+// number: the nine cells' counts are read together, then their buckets, then the
+// positions of a row of cells, and what the path progress needs is read at the
+// start.  One cell after the other (start, end, items, positions: 27 reads in a
+// row) took 22 us at 2,048 agents under ncu.  Blocks of 64 spread a small crowd over the
+// SMs.
+__global__ void __launch_bounds__(64, 8) k_collide_progress(MoverParams p) {
     if (*p.mv_count == 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.A) return;
     const ScenePar& sc = p.sc[p.agent_scene ? p.agent_scene[i] : 0];
     const float2 me = p.pos_mid[i];
-    float2 np = me;
     const int c = p.cell_of[i];
+    const bool moving = p.in_move[i];
+    const int L = p.path_len[i];
+    int si = p.step_idx[i];
+    const int sn = p.step_node[i];
+    const float2 step_pos = p.step_pos[i];
+    const int2* const heads = p.cell_head + (size_t)(*p.parity & 1) * p.cells;
+    float2 tri[3];  // the step's triangle
+    if (moving && sn >= 0 && sn < p.n) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) tri[k] = p.tri[3 * (size_t)sn + k];
+    }
+    float2 np = me;
     unsigned examined = 0;  // agents of the 3x3 cells read (the agent itself included)
     if (c >= 0) {
         const int lc = c - sc.cell_base;  // cell within the agent's scene
         const int cx = lc % sc.aw, cy = lc / sc.aw;
-        const int x0 = max(cx - 1, 0), x1 = min(cx + 1, sc.aw - 1);
-        const int y0 = max(cy - 1, 0), y1 = min(cy + 1, sc.ah - 1);
-        int ids[kMaxLocal];
-        float vxs[kMaxLocal], vys[kMaxLocal];
-        int cnt = 0;
-        bool overflow = false;
-        for (int yy = y0; yy <= y1; yy++)
-            for (int xx = x0; xx <= x1; xx++) {
-                const int cc = sc.cell_base + yy * sc.aw + xx;
-                examined += p.cell_start[cc + 1] - p.cell_start[cc];
-                for (int k = p.cell_start[cc], e = p.cell_start[cc + 1]; k < e; k++) {
-                    const int j = p.cell_items[k];
-                    if (j == i) continue;
-                    const float2 o = p.pos_mid[j];
-                    const float dx = GM_FSUB(me.x, o.x), dy = GM_FSUB(me.y, o.y);
-                    const float d2 = GM_FADD(GM_FMUL(dx, dx), GM_FMUL(dy, dy));
-                    if (!(d2 < sc.cd2)) continue;
-                    if (cnt >= kMaxLocal) {
-                        overflow = true;
-                        continue;
-                    }
-                    const float d = GM_FSQRT(d2);
-                    const float shift = GM_FSUB(sc.cd, d);
-                    const float vx = GM_FMUL(GM_FDIV(dx, d), shift);
-                    const float vy = GM_FMUL(GM_FDIV(dy, d), shift);
-                    // insertion keeps ids ascending
-                    int k2 = cnt++;
-                    while (k2 > 0 && ids[k2 - 1] > j) {
-                        ids[k2] = ids[k2 - 1];
-                        vxs[k2] = vxs[k2 - 1];
-                        vys[k2] = vys[k2 - 1];
-                        k2--;
-                    }
-                    ids[k2] = j;
-                    vxs[k2] = vx;
-                    vys[k2] = vy;
-                }
+        int2 h[9];
+        int4 b[9];
+        unsigned over = 0;  // cells with agents beyond their bucket
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            const int x = cx + k % 3 - 1, y = cy + k / 3 - 1;
+            const bool in = x >= 0 && x < sc.aw && y >= 0 && y < sc.ah;
+            h[k] = in ? heads[sc.cell_base + y * sc.aw + x] : make_int2(0, 0);
+        }
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            examined += h[k].x;
+            over |= (h[k].y != 0 ? 1u : 0u) << k;
+            b[k] = make_int4(-1, -1, -1, -1);
+            if (h[k].x > 0)
+                b[k] = *reinterpret_cast<const int4*>(p.bucket + kBucket * (size_t)(c + (k / 3 - 1) * sc.aw + k % 3 - 1));
+            // (entries beyond the count are a former frame's)
+            if (h[k].x < 2) b[k].y = -1;
+            if (h[k].x < 3) b[k].z = -1;
+            if (h[k].x < 4) b[k].w = -1;
+        }
+        Pushes ps;
+        auto meet = [&](int j, float2 o) {
+            const float dx = GM_FSUB(me.x, o.x), dy = GM_FSUB(me.y, o.y);
+            const float d2 = GM_FADD(GM_FMUL(dx, dx), GM_FMUL(dy, dy));
+            if (d2 < sc.cd2) ps.add(j, dx, dy, d2, sc.cd);
+        };
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            int id[12];
+            float2 o[12];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                id[4 * k] = b[3 * r + k].x;
+                id[4 * k + 1] = b[3 * r + k].y;
+                id[4 * k + 2] = b[3 * r + k].z;
+                id[4 * k + 3] = b[3 * r + k].w;
             }
+#pragma unroll
+            for (int k = 0; k < 12; k++) {
+                if (id[k] == i) id[k] = -1;
+                o[k] = id[k] >= 0 ? p.pos_mid[id[k]] : make_float2(0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < 12; k++)
+                if (id[k] >= 0) meet(id[k], o[k]);
+        }
+        for (; over; over &= over - 1) {
+            const int k = __ffs(over) - 1;
+            for (int j = heads[c + (k / 3 - 1) * sc.aw + k % 3 - 1].y - 1; j >= 0; j = p.next[j] - 1)
+                if (j != i) meet(j, p.pos_mid[j]);
+        }
         float sx = 0.f, sy = 0.f;
         int total = 0;
-        if (!overflow) {
-            for (int k = 0; k < cnt; k++) {
-                sx = GM_FADD(sx, vxs[k]);
-                sy = GM_FADD(sy, vys[k]);
+        if (!ps.overflow) {
+            for (int k = 0; k < ps.cnt; k++) {
+                sx = GM_FADD(sx, ps.vx[k]);
+                sy = GM_FADD(sy, ps.vy[k]);
             }
-            total = cnt;
+            total = ps.cnt;
         } else {
             // dense crowd: take contributors in ascending id by repeated minimum search
             int last = -1;
             for (;;) {
                 int best = 0x7fffffff;
                 float bvx = 0.f, bvy = 0.f;
-                for (int yy = y0; yy <= y1; yy++)
-                    for (int xx = x0; xx <= x1; xx++) {
-                        const int cc = sc.cell_base + yy * sc.aw + xx;
-                        for (int k = p.cell_start[cc], e = p.cell_start[cc + 1]; k < e; k++) {
-                            const int j = p.cell_items[k];
-                            if (j == i || j <= last || j >= best) continue;
-                            const float2 o = p.pos_mid[j];
-                            const float dx = GM_FSUB(me.x, o.x), dy = GM_FSUB(me.y, o.y);
-                            const float d2 = GM_FADD(GM_FMUL(dx, dx), GM_FMUL(dy, dy));
-                            if (!(d2 < sc.cd2)) continue;
-                            const float d = GM_FSQRT(d2);
-                            const float shift = GM_FSUB(sc.cd, d);
-                            best = j;
-                            bvx = GM_FMUL(GM_FDIV(dx, d), shift);
-                            bvy = GM_FMUL(GM_FDIV(dy, d), shift);
-                        }
+                auto look = [&](int j) {
+                    if (j == i || j <= last || j >= best) return;
+                    const float2 o = p.pos_mid[j];
+                    const float dx = GM_FSUB(me.x, o.x), dy = GM_FSUB(me.y, o.y);
+                    const float d2 = GM_FADD(GM_FMUL(dx, dx), GM_FMUL(dy, dy));
+                    if (!(d2 < sc.cd2)) return;
+                    const float d = GM_FSQRT(d2);
+                    const float shift = GM_FSUB(sc.cd, d);
+                    best = j;
+                    bvx = GM_FMUL(GM_FDIV(dx, d), shift);
+                    bvy = GM_FMUL(GM_FDIV(dy, d), shift);
+                };
+                for (int y = max(cy - 1, 0); y <= min(cy + 1, sc.ah - 1); y++)
+                    for (int x = max(cx - 1, 0); x <= min(cx + 1, sc.aw - 1); x++) {
+                        const int cc = sc.cell_base + y * sc.aw + x;
+                        const int2 q = heads[cc];
+                        for (int k = 0; k < min(q.x, kBucket); k++) look(p.bucket[kBucket * (size_t)cc + k]);
+                        for (int j = q.y - 1; j >= 0; j = p.next[j] - 1) look(j);
                     }
                 if (best == 0x7fffffff) break;
                 sx = GM_FADD(sx, bvx);
@@ -489,11 +521,9 @@ __global__ void k_collide_progress(MoverParams p) {
         if ((threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(p.stats + ST_NEIGHBOURS, (unsigned long long)tot);
     }
 
-    if (!p.in_move[i]) return;
+    if (!moving) return;
     // path progress
     const int* path = p.paths + (long long)i * p.path_stride;
-    const int L = p.path_len[i];
-    int si = p.step_idx[i];
     if (si == -1) {
         if (L < 1) {
             atomicOr(p.err, ERR_BOUNDS);
@@ -505,16 +535,14 @@ __global__ void k_collide_progress(MoverParams p) {
         p.step_pos[i] = p.waypoints ? p.waypoints[(long long)i * p.path_stride] : p.cen[nd];
         return;
     }
-    const int sn = p.step_node[i];
     if (sn < 0 || sn >= p.n) {
         atomicOr(p.err, ERR_BOUNDS);
         return;
     }
-    const bool inside = point_in_tri(np.x, np.y, p.tri[3 * sn], p.tri[3 * sn + 1], p.tri[3 * sn + 2]);
+    const bool inside = point_in_tri(np.x, np.y, tri[0], tri[1], tri[2]);
     bool at_point = false;  // path smoothing: the steering point reached
     if (p.waypoints && !inside) {
-        const float2 s = p.step_pos[i];
-        const float dx = GM_FSUB(s.x, np.x), dy = GM_FSUB(s.y, np.y);
+        const float dx = GM_FSUB(step_pos.x, np.x), dy = GM_FSUB(step_pos.y, np.y);
         at_point = GM_FSQRT(GM_FADD(GM_FMUL(dx, dx), GM_FMUL(dy, dy))) <= sc.arrive;
     }
     if (!inside && !at_point) return;
@@ -524,10 +552,9 @@ __global__ void k_collide_progress(MoverParams p) {
     } else {
         // a straight run to a funnel corner may cross thin corridor triangles
         // between two frames: skip every step that steers to the same point
-        const float2 s = p.step_pos[i];
         const float2* wp = p.waypoints + (long long)i * p.path_stride;
         int cur = p.cur_node[i];
-        while (si < L && wp[si].x == s.x && wp[si].y == s.y) cur = path[si++];
+        while (si < L && wp[si].x == step_pos.x && wp[si].y == step_pos.y) cur = path[si++];
         p.cur_node[i] = cur;
     }
     p.step_idx[i] = si;
@@ -731,13 +758,13 @@ inline int blocks_for(int n, int bt) { return (n + bt - 1) / bt; }
 
 void launch_compact(cudaStream_t s, int A, int* state, const int* cur, const int* targ, int P,
                     const CompactScenes& scn, int4* req, int* req_count, unsigned char* in_move, int* mv_count,
-                    int* work_ctr, int* hist, unsigned long long* stats) {
+                    int* parity, int* work_ctr, int* hist, unsigned long long* stats) {
     if (A <= kCompactThreads * kCompactRun)
         k_compact<<<1, kCompactThreads, 0, s>>>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count,
-                                                work_ctr, hist, stats);
+                                                parity, work_ctr, hist, stats);
     else
         k_compact_cluster<<<kCompactCluster, kCompactThreads, 0, s>>>(A, state, cur, targ, P, scn, req, req_count,
-                                                                      in_move, mv_count, work_ctr, hist, stats);
+                                                                      in_move, mv_count, parity, work_ctr, hist, stats);
 }
 
 void launch_apply_targets(cudaStream_t s, const int4* recs, int n, int* state, int* targ_node,
@@ -779,13 +806,7 @@ void launch_order_requests(cudaStream_t s, const int4* req_in, const int* req_co
 }
 
 void launch_move_bin(cudaStream_t s, const MoverParams& p) {
-    k_move_bin<<<blocks_for(p.A, 256), 256, 0, s>>>(p);
-}
-
-void launch_cell_scan(cudaStream_t s, const MoverParams& p) { k_cell_scan<<<1, 1024, 0, s>>>(p); }
-
-void launch_scatter(cudaStream_t s, const MoverParams& p) {
-    k_scatter<<<blocks_for(p.A, 256), 256, 0, s>>>(p);
+    k_move_bin<<<blocks_for(p.A, 128), 128, 0, s>>>(p);
 }
 
 void launch_funnel(cudaStream_t s, const MoverParams& p) {
@@ -794,7 +815,7 @@ void launch_funnel(cudaStream_t s, const MoverParams& p) {
 }
 
 void launch_collide_progress(cudaStream_t s, const MoverParams& p) {
-    k_collide_progress<<<blocks_for(p.A, 128), 128, 0, s>>>(p);
+    k_collide_progress<<<blocks_for(p.A, 64), 64, 0, s>>>(p);
 }
 
 }  // namespace gmapf_b200

@@ -222,6 +222,11 @@ OrderParams order_params(const Device& d, int2* keys) {
     return OrderParams{d.lm, d.lm_count, d.lm_max, d.order_hist, keys};
 }
 
+FrameWords frame_words(const Context& c) {
+    const Device& d = c.dev;
+    return FrameWords{c.h_step, reinterpret_cast<float*>(d.counters + 8), d.counters + CT_ERR};
+}
+
 CompactScenes compact_scenes(const Context& c) {
     const Device& d = c.dev;
     return CompactScenes{d.agent_scene, d.scene_abase, d.scene_P, d.scene_first};
@@ -407,10 +412,9 @@ int enqueue_frame(Context& c, bool timing, std::string& err) {
     Device& d = c.dev;
     cudaStream_t s = d.stream, s2 = d.stream2;
     if (timing) CK(cudaEventRecordWithFlags(d.ev[0], s, cudaEventRecordExternal));
-    CK(cudaMemsetAsync(d.counters + CT_ERR, 0, sizeof(int), s));
     launch_compact(s, c.A, d.state, d.cur, d.targ, c.cfg.PathFinderParallelAgents, compact_scenes(c), d.req,
                    d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_PARITY,
-                   d.counters + CT_WORK, d.order_hist, d.stats);
+                   d.counters + CT_WORK, d.order_hist, d.stats, frame_words(c));
     if (timing) CK(cudaEventRecordWithFlags(d.ev[1], s, cudaEventRecordExternal));
     CK(cudaEventRecord(d.ev[5], s));
     CK(cudaStreamWaitEvent(s2, d.ev[5], 0));
@@ -433,12 +437,7 @@ int enqueue_frame(Context& c, bool timing, std::string& err) {
     if (timing) CK(cudaEventRecordWithFlags(d.ev[3], s2, cudaEventRecordExternal));
     CK(cudaEventRecord(d.ev[6], s2));
     CK(cudaStreamWaitEvent(s, d.ev[6], 0));
-    if (c.A > 0) {
-        CK(cudaMemcpyAsync(c.h_pos_stage, d.pos, sizeof(float2) * c.A, cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(c.h_state_stage, d.state, sizeof(int) * c.A, cudaMemcpyDeviceToHost, s));
-    }
-    CK(cudaMemcpyAsync(c.h_small, d.counters, sizeof(int) * CT_COUNT, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(c.h_stats, d.stats, sizeof(unsigned long long) * ST_COUNT, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(c.h_frame, d.frame, d.frame_bytes, cudaMemcpyDeviceToHost, s));
     if (timing) CK(cudaEventRecordWithFlags(d.ev[4], s, cudaEventRecordExternal));
     return GMAPF_OK;
 }
@@ -511,11 +510,26 @@ int device_start(Context& c, std::string& err) {
 
     // agents
     const int A = c.A;
-    DALLOC(d.pos, A);
+    // what a frame brings back to the host, in one buffer and one copy:
+    // positions, states, counters, statistics
+    const size_t at_state = (sizeof(float2) * A + 15) & ~(size_t)15;
+    const size_t at_counters = (at_state + sizeof(int) * A + 15) & ~(size_t)15;
+    const size_t at_stats = at_counters + sizeof(int) * CT_COUNT;
+    d.frame_bytes = at_stats + sizeof(unsigned long long) * ST_COUNT;
+    DALLOC(d.frame, d.frame_bytes);
+    d.pos = reinterpret_cast<float2*>(d.frame);
+    d.state = reinterpret_cast<int*>(d.frame + at_state);
+    d.counters = reinterpret_cast<int*>(d.frame + at_counters);
+    d.stats = reinterpret_cast<unsigned long long*>(d.frame + at_stats);
+    CK(cudaMallocHost((void**)&c.h_frame, d.frame_bytes));
+    std::memset(c.h_frame, 0, d.frame_bytes);
+    c.h_pos_stage = reinterpret_cast<float2*>(c.h_frame);
+    c.h_state_stage = reinterpret_cast<int*>(c.h_frame + at_state);
+    c.h_small = reinterpret_cast<int*>(c.h_frame + at_counters);
+    c.h_stats = reinterpret_cast<unsigned long long*>(c.h_frame + at_stats);
     DALLOC(d.pos_mid, A);
     DALLOC(d.targ_pos, A);
     DALLOC(d.step_pos, A);
-    DALLOC(d.state, A);
     DALLOC(d.cur, A);
     DALLOC(d.targ, A);
     DALLOC(d.step_idx, A);
@@ -548,7 +562,6 @@ int device_start(Context& c, std::string& err) {
         DALLOC(d.waypoints, (size_t)std::max(1, A) * d.path_stride);
     }
     DALLOC(d.req, std::max(1, c.cfg.PathFinderParallelAgents));
-    DALLOC(d.counters, CT_COUNT);
     if (c.opt.order_by_estimate && c.opt.mode == GMAPF_MODE_BATCHED && n > 0 && nsc == 1) {
         // landmark hop distances for the longest-first request order
         std::vector<unsigned short> lm;
@@ -562,8 +575,6 @@ int device_start(Context& c, std::string& err) {
         DALLOC(d.req_sorted, std::max(1, c.cfg.PathFinderParallelAgents));
         DALLOC(d.req_keys, std::max(1, c.cfg.PathFinderParallelAgents));
     }
-    DALLOC(d.stats, ST_COUNT);
-
     std::vector<float2> tp(A);
     std::vector<int> minus(A, -1);
     for (int i = 0; i < A; i++) tp[i] = make_float2(c.m_targ[i].X, c.m_targ[i].Y);
@@ -609,13 +620,8 @@ int device_start(Context& c, std::string& err) {
     DALLOC(d.next, A);
 
     // pinned host staging
-    CK(cudaMallocHost((void**)&c.h_pos_stage, sizeof(float2) * std::max(1, A)));
-    CK(cudaMallocHost((void**)&c.h_state_stage, sizeof(int) * std::max(1, A)));
     CK(cudaMallocHost((void**)&c.h_dirty, sizeof(int4) * std::max(1, A)));
-    CK(cudaMallocHost((void**)&c.h_small, sizeof(int) * CT_COUNT));
-    CK(cudaMallocHost((void**)&c.h_stats, sizeof(unsigned long long) * ST_COUNT));
     CK(cudaMallocHost((void**)&c.h_step, sizeof(float) * 4));
-    std::memset(c.h_stats, 0, sizeof(unsigned long long) * ST_COUNT);
 
     int rc = alloc_search_state(c, err);
     if (rc) return rc;
@@ -659,9 +665,10 @@ void device_free(Context& c) {
     d.h_loc_pts = nullptr;
     d.h_loc_node = nullptr;
     d.loc_cap = 0;
-    void* hp[] = {c.h_pos_stage, c.h_state_stage, c.h_dirty, c.h_small, c.h_stats, c.h_step};
+    void* hp[] = {c.h_frame, c.h_dirty, c.h_step};
     for (void* p : hp)
         if (p) cudaFreeHost(p);
+    c.h_frame = nullptr;
     c.h_pos_stage = nullptr;
     c.h_state_stage = nullptr;
     c.h_dirty = nullptr;
@@ -690,8 +697,9 @@ int device_async_step(Context& c, float dt, std::string& err) {
         int rc = serve_before_frame(c, s, err);
         if (rc) return rc;
     }
-    c.h_step[0] = dt;  // each scene's step is speed * dt, rounded once (AgentsMover.h:63)
-    CK(cudaMemcpyAsync(d.counters + 8, c.h_step, sizeof(float), cudaMemcpyHostToDevice, s));
+    // each scene's step is speed * dt, rounded once (AgentsMover.h:63); the
+    // compaction reads it from the pinned word (no frame is in flight here)
+    c.h_step[0] = dt;
 
     if (c.opt.mode == GMAPF_MODE_BATCHED) {
         if (!d.graph_exec) {
@@ -704,10 +712,9 @@ int device_async_step(Context& c, float dt, std::string& err) {
         // plain: the reference's shape -- counts read back mid-frame
         const bool timing = c.cfg.IsProfiler != 0;
         if (timing) CK(cudaEventRecord(d.ev[0], s));
-        CK(cudaMemsetAsync(d.counters + CT_ERR, 0, sizeof(int), s));
         launch_compact(s, c.A, d.state, d.cur, d.targ, c.cfg.PathFinderParallelAgents, compact_scenes(c), d.req,
                        d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_PARITY,
-                       d.counters + CT_WORK, d.order_hist, d.stats);
+                       d.counters + CT_WORK, d.order_hist, d.stats, frame_words(c));
         c.launches += 1;
         CK(cudaMemcpyAsync(c.h_small, d.counters, sizeof(int) * CT_COUNT, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -736,12 +743,7 @@ int device_async_step(Context& c, float dt, std::string& err) {
             c.launches += 2 + (d.waypoints ? 1 : 0);
         }
         if (timing) CK(cudaEventRecord(d.ev[3], s));
-        if (c.A > 0) {
-            CK(cudaMemcpyAsync(c.h_pos_stage, d.pos, sizeof(float2) * c.A, cudaMemcpyDeviceToHost, s));
-            CK(cudaMemcpyAsync(c.h_state_stage, d.state, sizeof(int) * c.A, cudaMemcpyDeviceToHost, s));
-        }
-        CK(cudaMemcpyAsync(c.h_small, d.counters, sizeof(int) * CT_COUNT, cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(c.h_stats, d.stats, sizeof(unsigned long long) * ST_COUNT, cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(c.h_frame, d.frame, d.frame_bytes, cudaMemcpyDeviceToHost, s));
         if (timing) CK(cudaEventRecord(d.ev[4], s));
     }
     CK(cudaEventRecord(d.frame_done, s));
@@ -906,10 +908,9 @@ int device_search_batch(Context& c, const int* d_starts, const int* d_targets, i
         d.breq_cap = n;
     }
     CK(cudaMemsetAsync(d.counters + CT_ERR, 0, sizeof(int), s));
-    CK(cudaMemcpyAsync(c.h_stats, d.stats, sizeof(unsigned long long) * ST_COUNT, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    // the statistics so far: every call that changes them ends with reading them
     unsigned long long before[ST_COUNT];
-    std::memcpy(before, c.h_stats, sizeof(before));
+    std::memcpy(before, c.stats_prev, sizeof(before));
     launch_prepare_batch(s, d_starts, d_targets, n, c.map.n, d.breq, d.counters + CT_REQ,
                          d.counters + CT_WORK, d.order_hist, d.counters + CT_ERR);
     c.launches += 1;
@@ -952,8 +953,8 @@ int device_search_batch(Context& c, const int* d_starts, const int* d_targets, i
         }
     }
     CK(cudaEventRecord(d.ev[7], s));
-    CK(cudaMemcpyAsync(c.h_small, d.counters, sizeof(int) * CT_COUNT, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(c.h_stats, d.stats, sizeof(unsigned long long) * ST_COUNT, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(c.h_small, d.counters, sizeof(int) * CT_COUNT + sizeof(unsigned long long) * ST_COUNT,
+                       cudaMemcpyDeviceToHost, s));  // (the statistics follow the counters)
     CK(cudaStreamSynchronize(s));
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, d.ev[6], d.ev[7]));
@@ -972,7 +973,7 @@ int device_search_batch(Context& c, const int* d_starts, const int* d_targets, i
         out->ms_total_device = ms;
     }
     // keep the step's delta base consistent with the searches done here
-    for (int k = 0; k < ST_COUNT; k++) c.stats_prev[k] += c.h_stats[k] - before[k];
+    std::memcpy(c.stats_prev, c.h_stats, sizeof(before));
     const int e = c.h_small[CT_ERR];
     if (e != 0) {
         err = device_error_text(e);

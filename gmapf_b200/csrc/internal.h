@@ -172,9 +172,16 @@ struct CompactScenes {
     const int* P;
     int* first;
 };
+// words the compaction sets at a frame's start: the frame's dt (from pinned host
+// memory) and the error bits (cleared)
+struct FrameWords {
+    const float* dt_host;
+    float* dt;
+    int* err;
+};
 void launch_compact(cudaStream_t s, int A, int* state, const int* cur, const int* targ, int P,
                     const CompactScenes& scn, int4* req, int* req_count, unsigned char* in_move, int* mv_count,
-                    int* parity, int* work_ctr, int* hist, unsigned long long* stats);
+                    int* parity, int* work_ctr, int* hist, unsigned long long* stats, const FrameWords& words);
 void launch_apply_targets(cudaStream_t s, const int4* recs, int n, int* state, int* targ_node,
                           float2* targ_pos);
 // device-resident retargets of agents id_base + ids[k], ids[k] in [0, id_count)
@@ -286,6 +293,9 @@ struct Device {
     float2* cen = nullptr;
     float2* tri = nullptr;
     int *gstart = nullptr, *glist = nullptr, *degen = nullptr;
+    // positions, states, counters and statistics in one buffer (copied back as one)
+    unsigned char* frame = nullptr;
+    size_t frame_bytes = 0;
     // agents
     float2 *pos = nullptr, *pos_mid = nullptr, *targ_pos = nullptr, *step_pos = nullptr;
     int *state = nullptr, *cur = nullptr, *targ = nullptr, *step_idx = nullptr, *step_node = nullptr,
@@ -383,6 +393,7 @@ struct Context {
     std::vector<int> m_state, m_cur, m_targ_node;
     std::vector<gmapf_v2> m_targ;
     // pinned staging (allocated at start)
+    unsigned char* h_frame = nullptr;  // Device::frame on the host; the next four point into it
     float2* h_pos_stage = nullptr;
     int* h_state_stage = nullptr;
     int4* h_dirty = nullptr;

@@ -93,7 +93,7 @@ __device__ __forceinline__ int cluster_scan(int v, int* warp_tot, int* cluster_t
 template <int CL>
 __device__ __forceinline__ void compact(int A, int* state, const int* cur, const int* targ, int P, const CompactScenes& scn,
                                         int4* req, int* req_count, unsigned char* in_move, int* mv_count, int* parity,
-                                        int* work_ctr, int* hist, unsigned long long* stats) {
+                                        int* work_ctr, int* hist, unsigned long long* stats, const FrameWords& words) {
     __shared__ int warp_tot[32];
     __shared__ int cluster_tot[CL];
     const int tid = threadIdx.x;
@@ -101,6 +101,7 @@ __device__ __forceinline__ void compact(int A, int* state, const int* cur, const
     const bool scenes = scn.agent_scene != nullptr;
     static_assert(kOrderBuckets == kCompactThreads, "one bucket per thread");
     if (hist && rank == 0) hist[tid] = 0;  // the order's buckets
+    const float dt = tid == 0 && rank == 0 ? *reinterpret_cast<const volatile float*>(words.dt_host) : 0.f;
     int base_s = 0, base_m = 0, base_o = 0;  // before this step (the same on every thread)
     for (int b = 0; b < A; b += CL * kCompactThreads * kCompactRun) {
         const int i0 = b + (rank * kCompactThreads + tid) * kCompactRun;
@@ -186,6 +187,8 @@ __device__ __forceinline__ void compact(int A, int* state, const int* cur, const
         *mv_count = base_m;
         if (base_m > 0) *parity ^= 1;  // the mover runs: its grid takes turns
         *work_ctr = 0;
+        *words.dt = dt;
+        *words.err = 0;
         stats[ST_REQUESTS] += (unsigned long long)R;
         stats[ST_MOVING] += (unsigned long long)base_m;
     }
@@ -194,13 +197,13 @@ __device__ __forceinline__ void compact(int A, int* state, const int* cur, const
 
 #define COMPACT_ARGS                                                                                          \
     int A, int *state, const int *cur, const int *targ, int P, CompactScenes scn, int4 *req, int *req_count, \
-        unsigned char *in_move, int *mv_count, int *parity, int *work_ctr, int *hist, unsigned long long *stats
+        unsigned char *in_move, int *mv_count, int *parity, int *work_ctr, int *hist, unsigned long long *stats, FrameWords words
 __global__ void __launch_bounds__(kCompactThreads) k_compact(COMPACT_ARGS) {
-    compact<1>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, parity, work_ctr, hist, stats);
+    compact<1>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, parity, work_ctr, hist, stats, words);
 }
 __global__ void __cluster_dims__(kCompactCluster, 1, 1) __launch_bounds__(kCompactThreads)
     k_compact_cluster(COMPACT_ARGS) {
-    compact<kCompactCluster>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, parity, work_ctr, hist, stats);
+    compact<kCompactCluster>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, parity, work_ctr, hist, stats, words);
 }
 #undef COMPACT_ARGS
 
@@ -758,13 +761,13 @@ inline int blocks_for(int n, int bt) { return (n + bt - 1) / bt; }
 
 void launch_compact(cudaStream_t s, int A, int* state, const int* cur, const int* targ, int P,
                     const CompactScenes& scn, int4* req, int* req_count, unsigned char* in_move, int* mv_count,
-                    int* parity, int* work_ctr, int* hist, unsigned long long* stats) {
+                    int* parity, int* work_ctr, int* hist, unsigned long long* stats, const FrameWords& words) {
     if (A <= kCompactThreads * kCompactRun)
         k_compact<<<1, kCompactThreads, 0, s>>>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count,
-                                                parity, work_ctr, hist, stats);
+                                                parity, work_ctr, hist, stats, words);
     else
         k_compact_cluster<<<kCompactCluster, kCompactThreads, 0, s>>>(A, state, cur, targ, P, scn, req, req_count,
-                                                                      in_move, mv_count, parity, work_ctr, hist, stats);
+                                                                      in_move, mv_count, parity, work_ctr, hist, stats, words);
 }
 
 void launch_apply_targets(cudaStream_t s, const int4* recs, int n, int* state, int* targ_node,

@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
             int v = 0;
             if (lane == 0) v = atomicAdd(p.work_ctr, 1);
             r = __shfl_sync(kFull, v, 0);
-            R = *p.req_count_d;
+            R = p.starts ? p.req_count_h : *p.req_count_d;
         } else {
             if (iter > 0) break;
             r = req_base + slot;
@@ -309,14 +309,15 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
         }
         if (r >= R) break;
         // ring entries are rewritten by host copies over time: read past L1
-        const int4 rq = p.ring_cap > 0 ? __ldcg(p.req + ((p.ring_base + r) % p.ring_cap)) : p.req[r];
+        const int4 rq = p.starts         ? make_int4(-1, p.starts[r], p.targets[r], r)
+                        : p.ring_cap > 0 ? __ldcg(p.req + ((p.ring_base + r) % p.ring_cap)) : p.req[r];
         const int agent = rq.x, start = rq.y, target = rq.z, orow = rq.w;
         if (start < 0 || start >= n_nodes || target < 0 || target >= n_nodes || start == target) {
             const bool bad = start != target || start < 0 || start >= n_nodes;
             if (lane == 0) {  // bad request: not found; start == target: found, empty path
                 if (p.timeline) p.timeline[2 * (long long)orow] = p.timeline[2 * (long long)orow + 1] = global_timer_ns();
                 if (bad) atomicOr(p.err, ERR_BAD_REQUEST);
-                if (p.out_found) p.out_found[orow] = bad ? 0 : 1;
+                if (p.out_found) p.out_found[orow] = bad ? p.bad_code : 1;
                 if (p.out_len) p.out_len[orow] = 0;
                 if (agent >= 0 && p.ag_state) {
                     p.ag_state[agent] = GMAPF_AGENT_IDLE;
@@ -388,6 +389,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
         unsigned deg_sum = 0;
         int rounds = 0, expansions = 0, active = 2;  // active: nodes expanded by the coming round
         int claims = 2;                              // = entries of the claim log
+        bool cut = false;  // stopped by the round limit
         int found = 0, mS = -1, gS = 0, mT = -1, gT = 0;  // the meeting pair: log entries and depths
         int next_check = p.promote_rounds;  // placement 4: the round of the next room-in-block check
 
@@ -740,6 +742,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
             claims += nwin;
             if (rounds >= p.max_rounds) {  // still running after its last allowed round
                 if (lane == 0) atomicOr(p.err, ERR_ROUNDS);
+                cut = true;
                 return true;
             }
             reinterpret_cast<int4*>(seen)[lane] = make_int4(0, 0, 0, 0);
@@ -823,7 +826,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
         // results, agent update (PathFinder.h:268-289) and counters
         const unsigned ds = __reduce_add_sync(kFull, deg_sum);
         if (lane == 0) {
-            if (p.out_found) p.out_found[orow] = found;
+            if (p.out_found) p.out_found[orow] = cut ? p.cut_code : found;
             if (p.out_len) p.out_len[orow] = L;
             if (agent >= 0 && p.ag_state) {
                 // PathFinder.h:268-289: not found -> Idle with the path step
@@ -860,31 +863,34 @@ cudaError_t launch_t(cudaStream_t s, const SearchParams& p, int blocks, int bt, 
     return cudaGetLastError();
 }
 
-// (only ever raised, as for search.cu's kernel)
+// the kernel's dynamic shared-memory limit (only ever raised, as for search.cu's kernel)
 std::mutex g_smem_attr_mu;
 
 template <int T, int VM>
-int occupancy_t(int C, int bt, int bm_words, bool queues_global) {
+bool raise_smem_limit(int smem) {
     static int limit[64] = {};
-    if (bt > 256) return 0;  // the kernel's launch bounds
-    const size_t smem = smem_bytes(C, bt, bm_words, T, VM, queues_global);
-    if (smem > 227 * 1024) return 0;
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess) {
         cudaGetLastError();
-        return 0;
+        return false;
     }
-    {
-        std::lock_guard<std::mutex> lock(g_smem_attr_mu);
-        if ((int)smem > limit[device & 63]) {
-            if (cudaFuncSetAttribute(k_corridor_search<T, VM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem) != cudaSuccess) {
-                cudaGetLastError();
-                return 0;
-            }
-            limit[device & 63] = (int)smem;
+    std::lock_guard<std::mutex> lock(g_smem_attr_mu);
+    if (smem > limit[device & 63]) {
+        if (cudaFuncSetAttribute(k_corridor_search<T, VM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            return false;
         }
+        limit[device & 63] = smem;
     }
+    return true;
+}
+
+template <int T, int VM>
+int occupancy_t(int C, int bt, int bm_words, bool queues_global) {
+    if (bt > 256) return 0;  // the kernel's launch bounds
+    const size_t smem = smem_bytes(C, bt, bm_words, T, VM, queues_global);
+    if (smem > 227 * 1024 || !raise_smem_limit<T, VM>((int)smem)) return 0;
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_corridor_search<T, VM>, bt, smem) != cudaSuccess) {
         cudaGetLastError();
@@ -919,6 +925,21 @@ int occupancy_v(int T, int C, int bt, int bm_words, bool qg) {
 }
 
 }  // namespace
+
+size_t corridor_smem_bytes(int C, int bt, int bm_words, int T, int vm) {
+    return smem_bytes(C, bt, bm_words, T, vm, false);
+}
+
+bool corridor_full_smem(int T) {
+    switch (T) {
+        case 2: return raise_smem_limit<2, 1>(227 * 1024);
+        case 4: return raise_smem_limit<4, 1>(227 * 1024);
+        case 8: return raise_smem_limit<8, 1>(227 * 1024);
+        case 16: return raise_smem_limit<16, 1>(227 * 1024);
+        case 32: return raise_smem_limit<32, 1>(227 * 1024);
+        default: return false;
+    }
+}
 
 size_t corridor_queue_bytes(int C, int T) { return 4 * search_queue_words(C, T); }
 

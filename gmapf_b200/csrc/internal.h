@@ -108,6 +108,12 @@ struct SearchParams {
     int ring_cap;
     int ring_base;
     unsigned long long* done;
+    // corridor.cu only: requests straight from start and target arrays
+    // (req_count_h of them), and the found value of a bad request or of a search
+    // cut by the round limit (0 elsewhere)
+    const int* starts;
+    const int* targets;
+    int bad_code, cut_code;
     // diagnostics (batch searches): per output row, the GPU global timer when
     // a warp took the request [2 row] and when its results were written
     // [2 row + 1], or null
@@ -230,6 +236,10 @@ cudaError_t launch_corridor_search(cudaStream_t s, const SearchParams& p, int bl
                                    bool persistent, int req_base, int vm, int bm_words);
 int corridor_max_blocks_per_sm(int T, int C, int block_threads, int vm, int bm_words, bool queues_global);
 size_t corridor_queue_bytes(int C, int T);
+size_t corridor_smem_bytes(int C, int block_threads, int bm_words, int T, int vm);
+// lets visited placement 1 use all the shared memory of an SM on the current
+// device (so that later launches need no attribute call); false: a CUDA error
+bool corridor_full_smem(int T);
 
 // ------------------------------------------------------------------- host --
 

@@ -12,11 +12,14 @@
 //
 // That array (g_scratch, kScratchBytes) is a file-scope __device__ array:
 // every GPU that loads the library holds it until the process exits.  It
-// holds a small header (work counter, query counter) and the search records
-// of the concurrent request slots (32 bytes per navmesh triangle per slot).
+// holds a small header (work counter, query counter) and, by the navmesh's
+// size, either its edge rows and the claim logs of the concurrent request
+// slots (log form) or their search records (record form, 32 bytes per triangle
+// per slot).
 // Calls share it and it keeps the previous call's contents: the work counter
-// is cleared by each call, and records are stamped with a 64-bit query
-// number that never repeats (it would take centuries of queries to wrap), so
+// is cleared by each call, a claim log is read only where its search wrote it,
+// and records are stamped with a 64-bit query number that never repeats (it
+// would take centuries of queries to wrap), so
 // a stale record is never mistaken for a live one, whatever the earlier
 // calls' navmesh sizes were.  Two calls that overlap on the GPU (different
 // streams, or different host threads) race on it and give wrong results:
@@ -43,8 +46,16 @@ constexpr size_t kScratchBytes = size_t(64) << 20;  // 64 MiB per device
 constexpr size_t kHeaderBytes = 256;
 constexpr int kMaxDevices = 64;
 
-// header: 32-bit work counter at byte 0, 64-bit query counter at byte 8
-constexpr size_t kWorkOff = 0, kQueryOff = 8;
+// header: 32-bit work counter at byte 0, 64-bit query counter at byte 8, error
+// bits at 16 and counters from 64 (written, not read: results carry the codes)
+constexpr size_t kWorkOff = 0, kQueryOff = 8, kErrOff = 16, kStatsOff = 64;
+
+// Query stamps of the record form start here.  The log form leaves edge rows,
+// centroids and log entries in the same array; the upper word of a stamp, read
+// as any of those, would be an index or a depth of two billion or a signalling
+// NaN, which no arithmetic makes: what the one form leaves is never live to the
+// other.
+constexpr unsigned long long kFirstStamp = 0x7f900000ull << 32;
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
@@ -53,6 +64,7 @@ struct DeviceSetup {
     unsigned char* scratch = nullptr;  // device address of g_scratch
     int sms = 0;
     std::unordered_map<int, int> blocks_per_sm;  // (T, C) -> resident one-warp blocks per SM
+    bool log_ready[33] = {};                     // per T: the log form's kernel has its shared-memory limit
 };
 DeviceSetup g_setup[kMaxDevices];
 std::mutex g_setup_mu;
@@ -157,7 +169,7 @@ __global__ void __launch_bounds__(32) k_search_noalloc(NoAllocArgs a) {
             continue;
         }
         unsigned long long ep = 0;
-        if (lane == 0) ep = atomicAdd(qctr, 1ull) + 1ull;  // never repeats: stale records never match
+        if (lane == 0) ep = kFirstStamp + atomicAdd(qctr, 1ull) + 1ull;  // never repeats: stale records never match
         ep = __shfl_sync(kFull, ep, 0);
         const unsigned ep_lo = (unsigned)ep, ep_hi = (unsigned)(ep >> 32);
         const float2 cs = node_centroid(a.nodes, start), ct = node_centroid(a.nodes, target);
@@ -344,6 +356,79 @@ __global__ void __launch_bounds__(32) k_search_noalloc(NoAllocArgs a) {
     }
 }
 
+// ---- the log form: the search of corridor.cu in the same scratch array ----
+// Each call first lays out the navmesh as that kernel reads it (edge rows, third
+// candidates, centroids: 152 bytes per triangle), then searches with claim logs
+// of 16 bytes per triangle and slot and the visited bitmaps in shared memory.
+// On the 17,406-triangle maze that is 1.8 times the slots of the record form
+// (the slots that fit the array bound large navmeshes: 218 searches at a time
+// there), and shorter rounds: 2,048 queries at T=8, C=32 took 34.4 ms, now 9.1;
+// 37 on the 104,958-triangle maze at T=32, C=16 21.0, now 4.6; 2,048 between
+// rectangles (1,313 triangles) 0.148, now 0.118.  The record form stays for
+// navmeshes whose rows leave too few slots.
+
+// search.cu's SearchRow rules on caller-provided records: the neighbours up to
+// the first -1; ids outside the navmesh keep their slot but are no candidates
+__device__ __forceinline__ int leading(const gmapf_node& nd) {
+    int deg = 0;
+    while (deg < 3 && nd.NeibsIdx[deg] != -1) deg++;
+    return deg;
+}
+
+__global__ void k_noalloc_rows(const gmapf_node* nodes, int n, EdgeRow* rows, EdgeHalf* third, float2* cen) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= 4ll * n) return;
+    const int v = (int)(k >> 2), s = (int)(k & 3);
+    const gmapf_node& nd = nodes[v];
+    const int deg = leading(nd);
+    const int parent = s < deg ? nd.NeibsIdx[s] : -1;
+    EdgeRow o{{-1, (unsigned)deg << 4, 0.f, 0.f}, {-1, 0, 0.f, 0.f}};
+    EdgeHalf z{-1, 0, 0.f, 0.f};
+    int found = 0;
+    for (int j = 0; j < deg; j++) {
+        const int w = nd.NeibsIdx[j];
+        if (w == parent || w < 0 || w >= n) continue;
+        const gmapf_node& q = nodes[w];
+        int back = 3;
+        for (int b = leading(q) - 1; b >= 0; b--)
+            if (q.NeibsIdx[b] == v) back = b;
+        const float2 c = node_centroid(nodes, w);
+        if (found < 2) {
+            EdgeHalf& h = found == 0 ? o.x : o.y;
+            h.e = w << 2 | back;
+            h.info |= 1u << j;
+            h.x = c.x;
+            h.y = c.y;
+        } else {
+            z = EdgeHalf{w << 2 | back, 1u << j, c.x, c.y};
+            o.x.info |= kEdgeThird;
+        }
+        found++;
+    }
+    rows[k] = o;
+    if (s == 3) {
+        third[v] = z;
+        cen[v] = node_centroid(nodes, v);
+    }
+}
+
+struct LogLayout {
+    EdgeRow* rows;
+    EdgeHalf* third;
+    float2* cen;
+    int4* logs;
+    long long slots;  // 0: does not fit
+};
+LogLayout log_layout(unsigned char* scratch, int n) {
+    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t rows = up(kHeaderBytes), third = up(rows + sizeof(EdgeRow) * 4 * (size_t)n),
+                 cen = up(third + sizeof(EdgeHalf) * (size_t)n), logs = up(cen + sizeof(float2) * (size_t)n);
+    LogLayout l{reinterpret_cast<EdgeRow*>(scratch + rows), reinterpret_cast<EdgeHalf*>(scratch + third),
+                reinterpret_cast<float2*>(scratch + cen), reinterpret_cast<int4*>(scratch + logs), 0};
+    if (logs < kScratchBytes) l.slots = (long long)((kScratchBytes - logs) / (sizeof(int4) * (size_t)n));
+    return l;
+}
+
 size_t smem_per_warp(int T, int C) { return (size_t)4 * kEntry * T * (C + 3); }
 
 template <int T>
@@ -450,7 +535,10 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
         // this device; later calls make no CUDA calls besides the launch
         const int key = T * 1024 + C;
         auto it = ds->blocks_per_sm.find(key);
-        if (it == ds->blocks_per_sm.end()) it = ds->blocks_per_sm.emplace(key, occupancy_any(T, C)).first;
+        if (it == ds->blocks_per_sm.end()) {
+            it = ds->blocks_per_sm.emplace(key, occupancy_any(T, C)).first;
+            ds->log_ready[T] = ds->log_ready[T] || corridor_full_smem(T);
+        }
         per_sm = it->second;
     }
     if (per_sm <= 0) return fail(GMAPF_E_CAPACITY, "queues do not fit in shared memory for this T and C");
@@ -485,6 +573,43 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
     a.scratch = ds->scratch;
     a.slots = (int)slots;
     cudaError_t e;
+    // the log form, where its layout leaves as many slots as the record form has
+    // (or one for every query) and a warp's share fits in shared memory
+    const LogLayout lay = log_layout(ds->scratch, n_nodes);
+    const int bm_words = search_bitmap_words(n_nodes);
+    const size_t smem = corridor_smem_bytes(C, 32, bm_words, T, 1);
+    if (lay.slots >= std::min(by_mem, (long long)n_queries) && smem <= 227 * 1024 && ds->log_ready[T]) {
+        const long long per_sm_log = std::max<long long>(1, std::min<long long>(24, 228 * 1024 / (long long)(smem + 1024)));
+        const int blocks_log = (int)std::min({lay.slots, per_sm_log * ds->sms, (long long)n_queries});
+        k_noalloc_rows<<<(unsigned)((4ll * n_nodes + 255) / 256), 256, 0, s>>>(d_nodes, n_nodes, lay.rows, lay.third,
+                                                                              lay.cen);
+        SearchParams p{};
+        p.erow = lay.rows;
+        p.third = lay.third;
+        p.cen = lay.cen;
+        p.n = n_nodes;
+        p.starts = d_starts;
+        p.targets = d_targets;
+        p.req_count_h = n_queries;
+        p.T = T;
+        p.C = C;
+        p.K = heuristic_k;
+        p.log = lay.logs;
+        p.slots = blocks_log;
+        p.work_ctr = reinterpret_cast<int*>(ds->scratch + kWorkOff);
+        p.max_rounds = a.max_rounds;
+        p.paths = d_paths;
+        p.path_stride = path_stride;
+        p.out_found = d_found;
+        p.out_len = d_lens;
+        p.stats = reinterpret_cast<unsigned long long*>(ds->scratch + kStatsOff);
+        p.err = reinterpret_cast<int*>(ds->scratch + kErrOff);
+        p.bad_code = -1;
+        p.cut_code = -2;
+        e = launch_corridor_search(s, p, blocks_log, 32, true, 0, 1, bm_words);
+        if (e != cudaSuccess) return fail(GMAPF_E_CUDA, cudaGetErrorString(e));
+        return GMAPF_OK;
+    }
     switch (T) {
         case 2: e = run_t<2>(a, blocks, s); break;
         case 4: e = run_t<4>(a, blocks, s); break;

@@ -70,3 +70,40 @@ def test_queues_in_global_memory(oracle_mod, mode):
     rng = np.random.default_rng(6)
     s, t = (rng.integers(0, 2000, 300).astype(np.int32) for _ in range(2))
     check(oracle_mod, context(nodes, 32, 256, mode=mode), nodes, s, t, 32, 256)
+
+
+@pytest.mark.parametrize("T,Cap", [(2, 3), (8, 32), (16, 1), (32, 16)])
+def test_noalloc_log_form(lib, oracle_mod, T, Cap):
+    # caller-provided records: asymmetric lists, and neighbour ids outside the
+    # navmesh, which are no candidates (as if the triangle listed itself)
+    import ctypes as C
+    import torch
+    n = 1200
+    nodes = strip_map(n, 12, seed=9)
+    rng = np.random.default_rng(10)
+    same = nodes.copy()
+    for i in rng.integers(0, n, 150):
+        k = int(rng.integers(0, 3))
+        if nodes["NeibsIdx"][i, k] >= 0 and nodes["NeibsIdx"][i, k] != min(n - 1, i + 1):
+            nodes["NeibsIdx"][i, k] = [-9, n, 2**31 - 1][i % 3]
+            same["NeibsIdx"][i, k] = i
+    s, t = (rng.integers(0, n, 200).astype(np.int32) for _ in range(2))
+    s[7], t[9], t[11] = -1, n, s[11]
+    ok = np.ones(200, bool)
+    ok[[7, 9]] = False
+    of, ol, op, _ = oracle_mod.OMap(same).search_batch(np.where(ok, s, 0), np.where(ok, t, 1), T, Cap)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    d_nodes, d_s, d_t = dev(nodes.view(np.uint8)), dev(s), dev(t)
+    f, l = (torch.full((200,), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+    p = torch.full((200, n), -7, dtype=torch.int32, device="cuda")
+    for _ in range(2):
+        rc = lib.gmapf_search_batch_noalloc(d_nodes.data_ptr(), n, d_s.data_ptr(), d_t.data_ptr(), 200, T, Cap,
+                                            C.c_float(1.0), 0, f.data_ptr(), l.data_ptr(), p.data_ptr(), n,
+                                            C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        assert rc == 0
+        gf, gl, gp = f.cpu().numpy(), l.cpu().numpy(), p.cpu().numpy()
+        assert np.array_equal(gf[~ok], [-1, -1]) and np.array_equal(gl[~ok], [0, 0])
+        assert np.array_equal(gf[ok], of[ok]) and np.array_equal(gl[ok], ol[ok])
+        for i in np.nonzero(ok & (gf == 1))[0]:
+            assert np.array_equal(gp[i, :gl[i]], op[i, :gl[i]])

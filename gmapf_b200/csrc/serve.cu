@@ -371,27 +371,34 @@ int admit_and_launch(Context& c, Service& sv, std::string& err) {
             return GMAPF_E_DEVICE;
         }
     }
-    // the queries admitted since the last launch, as one batch on an idle stream
+    // the queries admitted since the last launch: one batch on an idle stream;
+    // more of them than a stream has slots go in equal parts to several, two of
+    // the idle ones left for later arrivals (4,096 queries at once between
+    // rectangles, T=8: one stream 339 us, six 75 us)
     if (sv.launched < sv.tail) {
-        int k = -1;
-        for (int j = 0; j < kStreams && k < 0; j++)
-            if (!sv.st_busy[j]) k = j;
-        if (k >= 0) {
-            const long long cnt = sv.tail - sv.launched;
-            sv.h_cnt[k] = (int)cnt;
+        int idle[kStreams], n_idle = 0;
+        for (int j = 0; j < kStreams; j++)
+            if (!sv.st_busy[j]) idle[n_idle++] = j;
+        const long long cnt = sv.tail - sv.launched;
+        const long long want = (cnt + sv.slots_per_stream - 1) / sv.slots_per_stream;
+        const int parts = (int)std::min<long long>(want, n_idle > 3 ? n_idle - 2 : std::min(n_idle, 1));
+        for (int q = 0; q < parts; q++) {
+            const int k = idle[q];
+            const long long part = (sv.tail - sv.launched) / (parts - q);
+            sv.h_cnt[k] = (int)part;
             cudaStream_t st = sv.st[k];
             if (sv.copy_recorded) SCK(cudaStreamWaitEvent(st, sv.copied, 0));
             SCK(cudaMemsetAsync(sv.d_wc + 2 * k, 0, sizeof(int), st));
             SCK(cudaMemcpyAsync(sv.d_wc + 2 * k + 1, sv.h_cnt + k, sizeof(int), cudaMemcpyHostToDevice, st));
             SearchParams sp = serve_params(c, sv, k);
             const int gpb = c.block_threads / 32;
-            const long long warps = std::min<long long>(cnt, sv.slots_per_stream);
+            const long long warps = std::min<long long>(part, sv.slots_per_stream);
             const int blocks = (int)((warps + gpb - 1) / gpb);
             SCK(launch_search(st, sp, blocks, c.block_threads, true, 0, c.dev.vm, c.dev.bm_words));
             SCK(cudaMemcpyAsync(sv.h_err + k, sv.d_err + k, sizeof(int), cudaMemcpyDeviceToHost, st));
             SCK(cudaEventRecord(sv.st_done[k], st));
             sv.st_busy[k] = true;
-            sv.launched = sv.tail;
+            sv.launched += part;
             sv.launches++;
             c.launches++;
         }
@@ -521,6 +528,21 @@ int serve_submit(Context& c, const int* ids, const gmapf_v2* pos, int n, const i
     // validate everything first: a rejected call queues nothing
     std::vector<Waiting> batch(n);
     const long long now = now_ns();
+    // A large burst's points are located on the device (targets, then the points
+    // under the agents; same rule): 8,192 points took 330 us here.
+    constexpr int kDeviceLocate = 1024;
+    std::vector<int> node;
+    if (n >= kDeviceLocate && !c.is_world) {
+        std::vector<gmapf_v2> pts(2 * (size_t)n);
+        for (int k = 0; k < n; k++) {
+            pts[k] = pos[k];
+            const int a = ids[k];
+            pts[n + k] = a >= 0 && a < c.A ? c.m_pos[a] : pos[k];
+        }
+        node.resize(pts.size());
+        const int rc = device_locate_points(c, pts.data(), (int)pts.size(), node.data(), err);
+        if (rc) return rc;
+    }
     for (int k = 0; k < n; k++) {
         const int a = ids[k];
         if (a < 0 || a >= c.A) {
@@ -528,14 +550,14 @@ int serve_submit(Context& c, const int* ids, const gmapf_v2* pos, int n, const i
             return GMAPF_E_INVALID_ARG;
         }
         const LocateGrid g = scene_grid(c, c.is_world ? scene_of_agent(c, a) : 0);
-        const int tnode = locate(g, pos[k].X, pos[k].Y);
+        const int tnode = node.empty() ? locate(g, pos[k].X, pos[k].Y) : node[k];
         if (tnode < 0) {
             err = "target pos (" + std::to_string(pos[k].X) + ", " + std::to_string(pos[k].Y) + ") is invalid";
             return GMAPF_E_INVALID_POS;
         }
         // the start: the triangle under the agent now (its last known triangle
         // if the position lies in none)
-        int start = locate(g, c.m_pos[a].X, c.m_pos[a].Y);
+        int start = node.empty() ? locate(g, c.m_pos[a].X, c.m_pos[a].Y) : node[n + k];
         if (start < 0) start = c.m_cur[a];
         batch[k] = Waiting{a, start, tnode, pos[k].X, pos[k].Y, arrival_ns ? (long long)arrival_ns[k] : now, 0};
     }

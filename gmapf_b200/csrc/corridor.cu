@@ -298,10 +298,17 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
         // ------------------------------------------------------------ fetch
         int r, R;
         if (persistent) {
-            int v = 0;
-            if (lane == 0) v = atomicAdd(p.work_ctr, 1);
-            r = __shfl_sync(kFull, v, 0);
             R = p.starts ? p.req_count_h : *p.req_count_d;
+            // a batch with a warp for every request: warp 0 of every block first, so
+            // that it spreads over the SMs, and no warp asks the counter
+            const int warps = (int)gridDim.x * wpb;
+            if (R <= warps && warps <= p.slots) {
+                r = iter == 0 ? wib * (int)gridDim.x + (int)blockIdx.x : R;
+            } else {
+                int v = 0;
+                if (lane == 0) v = atomicAdd(p.work_ctr, 1);
+                r = __shfl_sync(kFull, v, 0);
+            }
         } else {
             if (iter > 0) break;
             r = req_base + slot;

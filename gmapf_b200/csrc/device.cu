@@ -102,6 +102,7 @@ SearchParams search_params(Context& c) {
     p.epoch = d.epoch;
     p.log = d.form != FORM_RECORDS ? d.log : nullptr;
     p.queues = d.form == FORM_LOG_GLOBAL ? d.queues : nullptr;
+    p.full_pad = d.full_pad;
     p.slots = d.slots;
     p.gbm = d.gbm;
     p.work_ctr = d.counters + CT_WORK;
@@ -316,6 +317,11 @@ int pick_slots(Context& c, int& blocks, std::string& err) {
     d.form = best_form;
     d.slots = (int)best_slots;
     blocks = (int)(best_slots / (best_bt / 32));
+    // placement 4 on corridor maps: the shared memory that registers leave unused
+    // holds a bitmap more per block where it fits without a block less
+    d.full_pad = best_form != FORM_RECORDS && best_vm == 4 &&
+                 corridor_max_blocks_per_sm(c.T, c.C, best_bt, 4, d.bm_words, best_form == FORM_LOG_GLOBAL, true) >=
+                     search_max_blocks_per_sm(c.T, c.C, best_bt, 4, d.bm_words, best_form);
     // leave the kernel's shared-memory limit set for the chosen shape
     search_max_blocks_per_sm(c.T, c.C, best_bt, best_vm, d.bm_words, best_form);
     return GMAPF_OK;

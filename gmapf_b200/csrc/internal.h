@@ -88,6 +88,7 @@ struct SearchParams {
     unsigned* gbm;           // visited mode 3: bm_words 32-bit words per slot, global
     int* work_ctr;
     int max_rounds;
+    int full_pad;            // corridor.cu, visited placement 4: each block has room for one more bitmap
     int promote_rounds;      // visited placement 4: rounds before a search may move its bitmap into shared memory
     // outputs
     int* paths;              // row-major, path_stride ints per row
@@ -234,7 +235,8 @@ int search_max_blocks_per_sm(int T, int C, int block_threads, int vm, int bm_wor
 // corridor.cu (launch_search goes there when p.log is set)
 cudaError_t launch_corridor_search(cudaStream_t s, const SearchParams& p, int blocks, int block_threads,
                                    bool persistent, int req_base, int vm, int bm_words);
-int corridor_max_blocks_per_sm(int T, int C, int block_threads, int vm, int bm_words, bool queues_global);
+int corridor_max_blocks_per_sm(int T, int C, int block_threads, int vm, int bm_words, bool queues_global,
+                               bool full_pad);
 size_t corridor_queue_bytes(int C, int T);
 size_t corridor_smem_bytes(int C, int block_threads, int bm_words, int T, int vm);
 // lets visited placement 1 use all the shared memory of an SM on the current
@@ -333,6 +335,7 @@ struct Device {
     int* queues = nullptr;   // corridor maps: queues of the slots when they are not in shared memory
     size_t queue_cap = 0;    // its bytes
     int form = 0;            // SearchForm of the sized search
+    bool full_pad = false;   // corridor maps, placement 4: room for one more bitmap in each block
     int slots = 0;
     int vm = 2;                 // visited mode (1, 2 or 3; see launch_search)
     unsigned* gbm = nullptr;    // visited mode 3: slots x bm_words

@@ -839,7 +839,7 @@ size_t search_slot_bytes(int n_nodes, int vm, int bm_words, int form) {
 }
 
 int search_max_blocks_per_sm(int T, int C, int bt, int vm, int bm_words, int form) {
-    if (form != FORM_RECORDS) return corridor_max_blocks_per_sm(T, C, bt, vm, bm_words, form == FORM_LOG_GLOBAL);
+    if (form != FORM_RECORDS) return corridor_max_blocks_per_sm(T, C, bt, vm, bm_words, form == FORM_LOG_GLOBAL, false);
     switch (vm) {
         case 1: return occupancy_v<1>(T, C, bt, bm_words);
         case 2: return occupancy_v<2>(T, C, bt, 0);

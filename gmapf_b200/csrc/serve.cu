@@ -251,6 +251,7 @@ SearchParams serve_params(Context& c, Service& sv, int k) {
     p.epoch = sv.epoch;
     p.log = sv.log;
     p.queues = sv.queues;
+    p.full_pad = d.full_pad;
     p.gbm = sv.gbm;
     p.slot_base = k * sv.slots_per_stream;
     p.slots = sv.slots_per_stream;

@@ -413,6 +413,9 @@ void destroy_graph(Context& c) {
     c.dev.graph = nullptr;
 }
 
+// requests longest-first? (with a slot for each the order is of no use)
+bool frame_sorts(const Context& c) { return c.dev.lm && c.cfg.PathFinderParallelAgents > c.dev.slots; }
+
 // kernels of one frame on the two streams (batched form: captured)
 int enqueue_frame(Context& c, bool timing, std::string& err) {
     Device& d = c.dev;
@@ -426,7 +429,7 @@ int enqueue_frame(Context& c, bool timing, std::string& err) {
     CK(cudaStreamWaitEvent(s2, d.ev[5], 0));
     // search branch (requests longest-first when the landmark estimate is on)
     SearchParams sp = search_params(c);
-    if (d.lm) {
+    if (frame_sorts(c)) {
         launch_order_requests(s, d.req, d.counters + CT_REQ, std::max(1, c.cfg.PathFinderParallelAgents), d.req_sorted,
                               order_params(d, d.req_keys), c.map.n, d.slots);
         sp.req = d.req_sorted;
@@ -469,8 +472,7 @@ int capture_graph(Context& c, std::string& err) {
 }
 
 int kernels_per_frame(Context& c) {
-    const bool sorted = c.dev.lm && std::max(1, c.cfg.PathFinderParallelAgents) > c.dev.slots;
-    return 2 + (c.dev.lm ? 1 : 0) + (sorted ? 1 : 0) + (c.A > 0 ? 2 + (c.dev.waypoints ? 1 : 0) : 0);
+    return 2 + (frame_sorts(c) ? 2 : 0) + (c.A > 0 ? 2 + (c.dev.waypoints ? 1 : 0) : 0);
 }
 
 }  // namespace
@@ -922,10 +924,10 @@ int device_search_batch(Context& c, const int* d_starts, const int* d_targets, i
     c.launches += 1;
     SearchParams sp = search_params(c);
     sp.req = d.breq;
-    if (d.lm && n > 0) {
+    if (d.lm && n > d.slots) {
         launch_order_requests(s, d.breq, d.counters + CT_REQ, n, d.breq_sorted, order_params(d, d.breq_keys), c.map.n,
                               d.slots);
-        c.launches += n > d.slots ? 2 : 1;
+        c.launches += 2;
         sp.req = d.breq_sorted;
     }
     sp.paths = d_paths;

@@ -828,9 +828,8 @@ void launch_order_requests(cudaStream_t s, const int4* req_in, const int* req_co
                            const OrderParams& o, int n, int slots) {
     const int blocks = std::max(1, std::min(128, blocks_for(most, 256)));
     k_order_keys<<<blocks, 256, 0, s>>>(req_in, req_count, req_out, o.keys, o.hist, o.lm, o.L, n, o.lm_max, slots);
-    if (most > slots)
-        k_order_place<<<std::min(32, blocks_for(most, 1024)), 1024, 0, s>>>(req_in, req_count, req_out, o.keys, o.hist,
-                                                                           slots);
+    k_order_place<<<std::min(32, blocks_for(most, 1024)), 1024, 0, s>>>(req_in, req_count, req_out, o.keys, o.hist,
+                                                                       slots);
 }
 
 void launch_move_bin(cudaStream_t s, const MoverParams& p) {

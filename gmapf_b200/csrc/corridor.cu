@@ -475,10 +475,10 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
                 g[j] = c[j].e >= 0;
                 // the candidate's own edge row, for the round that expands it
                 copy_edge_row(rows + 2 * (j * 32 + lane), p.erow, c[j].e);
-                const unsigned bit = 1u << (n[j] & 31);
-                unsigned taken = 0;
-                if (g[j]) taken = atomicOr(seen + ((n[j] >> 5) & (kSeenWords - 1)), bit) & bit;
-                const int v = g[j] ? visited(n[j]) : 0;
+                // (lanes without a candidate set no bit, each in its own word: no branch)
+                const unsigned bit = g[j] ? 1u << (n[j] & 31) : 0u;
+                const unsigned taken = atomicOr(seen + (g[j] ? (n[j] >> 5) & (kSeenWords - 1) : lane), bit) & bit;
+                const int v = SMX ? (g[j] ? bm_get(bmx, n[j]) : 0) : bm_bits(ld_word_if(bmx + (n[j] >> 4), g[j]), n[j]);
                 cross[j] = v != 0 && (v >> 1) != du;
                 g[j] = g[j] && v == 0;
                 s[j] = g[j] && taken;

@@ -42,12 +42,23 @@ __device__ __forceinline__ void ld_edge_row(const EdgeRow* rows, int k, EdgeHalf
 }
 
 // the row into shared memory, asynchronously; copies_done waits for this thread's copies
+// a word through L2, 0 (and no access) without `on`
+__device__ __forceinline__ unsigned ld_word_if(const unsigned* p, bool on) {
+    unsigned w;
+    asm volatile("{ .reg .pred q; setp.ne.s32 q, %2, 0; mov.b32 %0, 0; @q ld.global.cg.b32 %0, [%1]; }"
+                 : "=&r"(w)
+                 : "l"(p), "r"((int)on)
+                 : "memory");
+    return w;
+}
+
+// (k < 0: zeros, and nothing is read)
 __device__ __forceinline__ void copy_edge_row(EdgeHalf* to, const EdgeRow* rows, int k) {
-    if (k < 0) return;
     const unsigned d = (unsigned)__cvta_generic_to_shared(to);
-    const EdgeRow* from = rows + k;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(&from->x) : "memory");
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16), "l"(&from->y) : "memory");
+    const EdgeRow* from = rows + max(k, 0);
+    const int bytes = k < 0 ? 0 : 16;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(&from->x), "r"(bytes) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d + 16), "l"(&from->y), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 

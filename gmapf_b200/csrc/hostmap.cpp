@@ -194,6 +194,8 @@ int corridor_levels(const HostMap& m, const std::vector<SceneInfo>& scenes) {
                 lv = d[src] + 1;
                 cnt = (long long)q.size();
             }
+            // the second wave has at most twice the levels: often the first one tells
+            if ((lv >= 256 && cnt <= 16 * lv) || cnt > 32 * lv) break;
         }
         levels += lv;
         nodes += cnt;

@@ -54,7 +54,7 @@ int search_promote_rounds(const Context& c) { return c.opt.promote_rounds > 0 ? 
 namespace {
 
 // device counters: [8] holds the frame's dt as a float
-enum Counter { CT_REQ = 0, CT_MOVE = 1, CT_WORK = 2, CT_ERR = 3, CT_ERR_TARGETS = 4, CT_PARITY = 9, CT_COUNT = 16 };
+enum Counter { CT_REQ = 0, CT_MOVE = 1, CT_WORK = 2, CT_ERR = 3, CT_ERR_TARGETS = 4, CT_PARITY = 9 /* and 10 */, CT_COUNT = 16 };
 
 template <class T>
 int dalloc(Context& c, T** p, size_t count, std::string& err) {

@@ -156,7 +156,7 @@ struct MoverParams {
     // agent grid (all scenes' cells, global ids)
     int cells;
     int* cell_of;
-    const int* parity; // whose turn of the two copies of cell_head it is
+    int* parity;       // [0] whose turn of the two copies of cell_head it is, [1] the copy has been used
     int2* cell_head;   // 2 x cells: agents in the cell, list of those beyond its bucket
     int* bucket;       // 4 x cells: the first agents of a cell
     int* next;         // A: the lists

@@ -185,7 +185,10 @@ __device__ __forceinline__ void compact(int A, int* state, const int* cur, const
         const int R = scenes ? base_o : (base_s < P ? base_s : P);
         *req_count = R;
         *mv_count = base_m;
-        if (base_m > 0) *parity ^= 1;  // the mover runs: its grid takes turns
+        if (parity[1]) {  // the mover has used its grid since: the other copy's turn
+            parity[0] ^= 1;
+            parity[1] = 0;
+        }
         *work_ctr = 0;
         *words.dt = dt;
         *words.err = 0;
@@ -314,7 +317,8 @@ __global__ void __launch_bounds__(1024) k_order_place(const int4* req_in, const 
 // scan over the cells and no second pass to place the agents (k_cell_scan and
 // k_scatter took 4 + 4 us at 2,048 agents, 39 + 4 us at 24,000 in 64 scenes).
 // Two copies of the counts take turns, so that a frame's binning clears the
-// other frame's without a launch of its own; *p.parity says whose turn it is.
+// other frame's without a launch of its own; *p.parity says whose turn it is (the
+// compaction switches it once the collision pass has marked the copy as used).
 constexpr int kBucket = 4;
 
 // move (AgentsMover.h:51-71) fused with the binning
@@ -397,6 +401,7 @@ __global__ void __launch_bounds__(64, 8) k_collide_progress(MoverParams p) {
     if (*p.mv_count == 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.A) return;
+    if (i == 0) p.parity[1] = 1;
     const ScenePar& sc = p.sc[p.agent_scene ? p.agent_scene[i] : 0];
     const float2 me = p.pos_mid[i];
     const int c = p.cell_of[i];
@@ -465,7 +470,9 @@ __global__ void __launch_bounds__(64, 8) k_collide_progress(MoverParams p) {
         }
         for (; over; over &= over - 1) {
             const int k = __ffs(over) - 1;
-            for (int j = heads[c + (k / 3 - 1) * sc.aw + k % 3 - 1].y - 1; j >= 0; j = p.next[j] - 1)
+            const int2 q = heads[c + (k / 3 - 1) * sc.aw + k % 3 - 1];
+            int left = q.x - kBucket;  // (the count bounds the walk)
+            for (int j = q.y - 1; j >= 0 && left > 0; j = p.next[j] - 1, left--)
                 if (j != i) meet(j, p.pos_mid[j]);
         }
         float sx = 0.f, sy = 0.f;
@@ -499,7 +506,8 @@ __global__ void __launch_bounds__(64, 8) k_collide_progress(MoverParams p) {
                         const int cc = sc.cell_base + y * sc.aw + x;
                         const int2 q = heads[cc];
                         for (int k = 0; k < min(q.x, kBucket); k++) look(p.bucket[kBucket * (size_t)cc + k]);
-                        for (int j = q.y - 1; j >= 0; j = p.next[j] - 1) look(j);
+                        int left = q.x - kBucket;
+                        for (int j = q.y - 1; j >= 0 && left > 0; j = p.next[j] - 1, left--) look(j);
                     }
                 if (best == 0x7fffffff) break;
                 sx = GM_FADD(sx, bvx);

@@ -500,13 +500,6 @@ int device_start(Context& c, std::string& err) {
     DALLOC(d.glist, m.glist.size());
     DALLOC(d.degen, m.degen.size());
     CK(cudaMemcpyAsync(d.rows, m.rows.data(), sizeof(SearchRow) * n, cudaMemcpyHostToDevice, d.stream));
-    d.corridor_levels = corridor_levels(m, c.scenes);
-    if (d.corridor_levels >= 64) {
-        DALLOC(d.erow, 4 * (size_t)n);
-        DALLOC(d.third, n);
-        launch_edge_rows(d.stream, d.rows, n, d.erow, d.third);
-        CK(cudaGetLastError());
-    }
     CK(cudaStreamSynchronize(d.stream));
     CK(cudaMemcpy(d.cen, m.cen.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d.tri, m.tri.data(), sizeof(float2) * 3 * n, cudaMemcpyHostToDevice));
@@ -630,6 +623,21 @@ int device_start(Context& c, std::string& err) {
     // pinned host staging
     CK(cudaMallocHost((void**)&c.h_dirty, sizeof(int4) * std::max(1, A)));
     CK(cudaMallocHost((void**)&c.h_step, sizeof(float) * 4));
+
+    // long corridors: the edge rows (144 bytes per triangle; a directed edge is an
+    // int) where they take little of what is left, else search.cu serves all maps
+    d.corridor_levels = 0;
+    if (n > 0 && n <= (1 << 24)) {
+        size_t freeb = 0, totalb = 0;
+        CK(cudaMemGetInfo(&freeb, &totalb));
+        if (144 * (double)n <= 0.05 * (double)freeb) d.corridor_levels = corridor_levels(m, c.scenes);
+    }
+    if (d.corridor_levels >= 64) {
+        DALLOC(d.erow, 4 * (size_t)n);
+        DALLOC(d.third, n);
+        launch_edge_rows(d.stream, d.rows, n, d.erow, d.third);
+        CK(cudaGetLastError());
+    }
 
     int rc = alloc_search_state(c, err);
     if (rc) return rc;

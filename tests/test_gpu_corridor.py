@@ -107,3 +107,41 @@ def test_noalloc_log_form(lib, oracle_mod, T, Cap):
         assert np.array_equal(gf[ok], of[ok]) and np.array_equal(gl[ok], ol[ok])
         for i in np.nonzero(ok & (gf == 1))[0]:
             assert np.array_equal(gp[i, :gl[i]], op[i, :gl[i]])
+
+
+def test_scene_batch_and_serving_on_corridors(oracle_mod):
+    # two winding corridors stepped as one batch, then one of them served: the
+    # corridor kernel with global ids, and on the serving streams
+    from test_gpu_frame_kernels import inside, pair, step_and_compare, target, winding_map
+    maps = [winding_map(9, 40, 8.0), winding_map(20, 18, 9.0)]
+    rng = np.random.default_rng(12)
+    sets = []
+    for nodes in maps:
+        g, ow = pair(oracle_mod, nodes, inside(nodes, 50, rng), 8, 16, 50, radius=1.0)
+        sets.append((g, ow, nodes))
+    batch = G.SceneBatch([g for g, _, _ in sets])
+    batch.ManualStart()
+    assert batch.world.search_shape()["T"] == 8
+    for frame in range(4):
+        if frame % 2 == 0:
+            for g, ow, nodes in sets:
+                target(g, ow, np.arange(50, dtype=np.int32), inside(nodes, 50, rng))
+        batch.AsyncStep(0.5)
+        batch.WaitStepEnd()
+        for g, ow, _ in sets:
+            ow.step(0.5, 4)
+            d, o = g.debug_agents(), ow.get()
+            for k in ("state", "path_len", "step_idx"):
+                assert np.array_equal(d[k], o[k]), k
+    nodes = maps[1]
+    start, goal = inside(nodes, 1500, rng), inside(nodes, 1500, rng)
+    g, _ = pair(oracle_mod, nodes, start, 8, 16, 1500, radius=0.1)
+    g.serve_start(0)
+    g.serve_submit(np.arange(1500, dtype=np.int32), goal)
+    g.serve_drain()
+    om = oracle_mod.OMap(g.map_nodes())
+    s, t = om.locate_batch(start), om.locate_batch(goal)
+    f, l, p, _ = om.search_batch(s, t, 8, 16)
+    for a in range(0, 1500, 37):
+        gf, gl, gp = g.serve_result(a)
+        assert gf == f[a] and gl == l[a] and np.array_equal(gp, p[a, :l[a]])

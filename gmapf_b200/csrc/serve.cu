@@ -122,6 +122,7 @@ struct Service {
     cudaEvent_t st_done[kStreams] = {};
     bool st_busy[kStreams] = {};
     int slots_per_stream = 0;
+    bool room = false;     // the searches leave room on every SM for other kernels
     int* d_wc = nullptr;   // per stream: work counter, query count
     int* h_cnt = nullptr;  // pinned: per stream, the batch's query count
     int* d_err = nullptr;  // per stream: device-side error bits
@@ -444,6 +445,7 @@ int serve_start(Context& c, int max_in_flight, std::string& err) {
     // the drain launch is persistent while queries keep coming: leave one
     // block per SM for the frames' own kernels
     const int drain_per_sm = per_sm > 1 ? per_sm - 1 : 1;
+    sv.room = per_sm > 1;
     long long slots = std::min<long long>((long long)sms * drain_per_sm * gpb, (long long)(0.25 * freeb / per_slot));
     // split over the streams, whole blocks each
     const long long per_stream = (slots / kStreams / gpb) * gpb;
@@ -533,7 +535,7 @@ int serve_submit(Context& c, const int* ids, const gmapf_v2* pos, int n, const i
     // under the agents; same rule): 8,192 points took 330 us here.
     constexpr int kDeviceLocate = 1024;
     std::vector<int> node;
-    if (n >= kDeviceLocate && !c.is_world) {
+    if (n >= kDeviceLocate && !c.is_world && sv.room) {
         std::vector<gmapf_v2> pts(2 * (size_t)n);
         for (int k = 0; k < n; k++) {
             pts[k] = pos[k];

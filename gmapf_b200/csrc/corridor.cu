@@ -39,20 +39,66 @@ namespace gmapf_b200 {
 
 namespace {
 
+// The claim log: entry i of a search is its i-th claim, {directed edge, G<<1|dir,
+// parent's entry, jump ancestor's entry}; the jump ancestor is the nearest
+// proper ancestor whose depth (G) is a multiple of kJumpDepth (-1: a root).
+constexpr int kJumpDepth = 32;
+
+// An entry as it is: one 16-byte access.
+struct WideLog {
+    using Entry = int4;
+    int4* p;
+    __device__ __forceinline__ int4 get(int i) const { return __ldcg(p + i); }
+    __device__ __forceinline__ int2 claim(int i) const { return __ldcg(reinterpret_cast<const int2*>(p + i)); }
+    __device__ __forceinline__ int edge(int i) const { return __ldcg(&p[i].x); }
+    __device__ __forceinline__ int key(int i) const { return __ldcg(&p[i].y); }
+    __device__ __forceinline__ int jump(int i) const { return __ldcg(&p[i].w); }
+    __device__ __forceinline__ void put(int i, int4 q) const { __stcg(p + i, q); }
+};
+
+// In 8 bytes, for maps of at most kPackedLogNodes triangles: edge 17 bits, G<<1|dir
+// 16 (a depth is below the claims), parent + 1 and jump + 1 15 each (an ancestor is
+// an earlier claim).  Twice the searches in a fixed scratch array (searches without
+// allocation).  Where memory is not the limit the wide entry costs fewer
+// instructions: 64x64-cell maze, placement 1, 16,384 searches at T=4 14.5 against
+// 14.9 ms, T=8 6.9 against 7.0, 37 searches 0.575 against 0.603; at T=32 the packed
+// one is 0-6% faster, within what its runs differ by.
+struct PackedLog {
+    using Entry = uint2;
+    uint2* p;
+    static __device__ __forceinline__ int4 unpack(uint2 v) {
+        return make_int4((int)(v.x & 0x1ffffu), (int)(v.y & 0xffffu), (int)(v.x >> 17) - 1, (int)(v.y >> 16) - 1);
+    }
+    __device__ __forceinline__ int4 get(int i) const { return unpack(__ldcg(p + i)); }
+    __device__ __forceinline__ int2 claim(int i) const {
+        const int4 q = get(i);
+        return make_int2(q.x, q.y);
+    }
+    __device__ __forceinline__ int edge(int i) const { return get(i).x; }
+    __device__ __forceinline__ int key(int i) const { return get(i).y; }
+    __device__ __forceinline__ int jump(int i) const { return get(i).w; }
+    __device__ __forceinline__ void put(int i, int4 q) const {
+        __stcg(p + i, make_uint2((unsigned)q.x | (unsigned)(q.z + 1) << 17, (unsigned)q.y | (unsigned)(q.w + 1) << 16));
+    }
+};
+static_assert(kPackedLogNodes <= 1 << 15, "PackedLog: an edge has 17 bits, an entry 15");
+
 // bounded push (CuQueue.h:33-63 with the (F,G,id) order) into a ring holding
 // at most cap entries, kept in descending order (minimum at the tail)
 // (entries keep their place in the claim log; their directed edge is read from
 // there only to break a tie of F and G)
-__device__ __forceinline__ bool entry_less(const int4* log, int2 a, int ia, float F, int gd, int e, bool flip) {
+template <class LG>
+__device__ __forceinline__ bool entry_less(LG log, int2 a, int ia, float F, int gd, int e, bool flip) {
     const float fa = __int_as_float(a.x);
     if (fa != F) return flip ? F < fa : fa < F;
     if ((a.y | 1) != (gd | 1)) return flip ? (gd | 1) < (a.y | 1) : (a.y | 1) < (gd | 1);
-    const int ea = __ldcg(&log[ia].x);
+    const int ea = log.edge(ia);
     return flip ? e < ea : ea < e;
 }
 
-__device__ __forceinline__ void ring_push(const Ring& r, const int4* log, int& beg, int& size, int cap, float F, int gd,
-                                          int e, int id) {
+template <class LG>
+__device__ __forceinline__ void ring_push(const Ring& r, LG log, int& beg, int& size, int cap, float F, int gd, int e,
+                                          int id) {
     if (cap <= 0) return;
     if (size == cap) {
         const int k0 = r.at(beg);
@@ -89,22 +135,18 @@ __host__ __device__ __forceinline__ size_t corridor_frontier_words(int T) {
     return (size_t)4 * 3 * T + kSeenWords + 8 * corridor_staged_rows(T) + ((3 * T + 15) / 16) * 4;
 }
 
-// The claim log: entry i of a search is its i-th claim, {directed edge, G<<1|dir,
-// parent's entry, jump ancestor's entry}; the jump ancestor is the nearest
-// proper ancestor whose depth (G) is a multiple of kJumpDepth (-1: a root).
-constexpr int kJumpDepth = 32;
-
 // The log entry and G<<1|dir of node n (claimed by this search), newest first;
 // -1 if none.  The other side's claim of the meeting node can be old (a queue
 // dropped it): on the 160x160 maze 9-15 thousand claims back on average.
-__device__ __noinline__ int2 find_claim(const int4* log, int claims, int n, int lane) {
+template <class LG>
+__device__ __noinline__ int2 find_claim(LG log, int claims, int n, int lane) {
     constexpr int U = 8;  // 256 entries per step, all reads in flight
     for (int top = claims; top > 0; top -= 32 * U) {
         int2 q[U];
 #pragma unroll
         for (int j = 0; j < U; j++) {
             const int i = top - 1 - (j * 32 + lane);
-            q[j] = i >= 0 ? __ldcg(reinterpret_cast<const int2*>(log + i)) : make_int2(-1, 0);
+            q[j] = i >= 0 ? log.claim(i) : make_int2(-1, 0);
         }
         int hit = -1, gd = 0;
 #pragma unroll
@@ -130,13 +172,14 @@ __device__ __noinline__ int2 find_claim(const int4* log, int claims, int n, int 
 // dependent reads.
 // A short search's log is read into shared memory (buf, cap entries) first and
 // followed there.
-__device__ __forceinline__ void walk_path(const int4* log, int claims, int2* buf, int cap, int* out, int mS, int gS,
+template <class LG>
+__device__ __forceinline__ void walk_path(LG log, int claims, int2* buf, int cap, int* out, int mS, int gS,
                                           int mT, int gT, int lane, int* err) {
     if (claims <= cap) {
         __syncwarp();
 #pragma unroll 4
         for (int i = lane; i < claims; i += 32) {
-            const int4 q = __ldcg(log + i);
+            const int4 q = log.get(i);
             buf[i] = make_int2(q.x >> 2, q.z);
         }
         __syncwarp();
@@ -163,7 +206,7 @@ __device__ __forceinline__ void walk_path(const int4* log, int claims, int2* buf
         int x = lane == 0 ? mS : mT;
         kc = g >= 1 ? (g - 1) / kJumpDepth : 0;
         for (int k = kc; k >= 1 && !bad; k--) {
-            x = __ldcg(&log[x].w);  // the nearest ancestor at a multiple of D: depth k*D
+            x = log.jump(x);  // the nearest ancestor at a multiple of D: depth k*D
             bad = x < 0 || x >= claims;
             if (!bad) out[path_pos(lane, k * kJumpDepth, gS, gT)] = x;
         }
@@ -219,7 +262,7 @@ __device__ __forceinline__ void walk_path(const int4* log, int claims, int2* buf
                     b[j] = 0;
                     continue;
                 }
-                q[j] = __ldcg(log + x[j]);
+                q[j] = log.get(x[j]);
             }
 #pragma unroll
             for (int j = 0; j < W; j++) {
@@ -254,7 +297,7 @@ size_t smem_bytes(int C, int bt, int bm_words, int T, int vm, bool queues_global
 // still running at a batch's tail moves into the shared memory of its block's
 // finished warps, as in search.cu).  A bit set by one thread is seen by the
 // others after the next __syncwarp.
-template <int T, int VM>
+template <int T, int VM, class LG>
 __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int persistent, int req_base, int bm_words) {
     constexpr bool SMEMV = VM == 1;  // bitmap in shared memory
     extern __shared__ __align__(16) unsigned char smem[];
@@ -298,7 +341,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
 
     if (slot >= p.slots) return;  // whole warps
     if (VM == 4) bm = p.gbm + (size_t)(p.slot_base + slot) * bm_words;
-    int4* log = p.log + (size_t)(p.slot_base + slot) * n_nodes;
+    const LG log{static_cast<typename LG::Entry*>(p.log) + (size_t)(p.slot_base + slot) * n_nodes};
     const unsigned lt_mask = (1u << lane) - 1u;
 
     for (int iter = 0;; iter++) {
@@ -391,7 +434,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
             e = (node << 2) | 3;
             at = k;
             if (lane < 2) {
-                __stcg(log + lane, make_int4(e, gd, -1, -1));
+                log.put(lane, make_int4(e, gd, -1, -1));
                 bm_set<SMEMV>(bm, node, gd);
             }
         }
@@ -436,14 +479,14 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
             auto write_claim = [&](int i, int en, float cx, float cy) {
                 const float F = GM_FADD(gf, GM_FMUL(dist_sqr(cx, cy, farx, fary), K));
                 fr[i] = make_int4(__float_as_int(F), ngd, en, cjump);
-                __stcg(log + (claims + i), make_int4(en, ngd, at, cjump));
+                log.put(claims + i, make_int4(en, ngd, at, cjump));
             };
 
             // the search's end: node mn, log entry `other` (-1: look for it), met from log entry mat with key mgd
             auto finish = [&](int mat, int mgd, int mn, int other) {
                 int ogd;
                 if (other >= 0) {
-                    ogd = __ldcg(log + other).y;
+                    ogd = log.key(other);
                 } else {
                     const int2 f = find_claim(log, claims, mn, lane);
                     other = f.x;
@@ -749,7 +792,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
                         top.F = __int_as_float(w.x);
                         top.gd = w.y;
                         top.at = ring.id()[k];
-                        const int4 c = __ldcg(log + top.at);
+                        const int4 c = log.get(top.at);
                         top.e = c.x;
                         top.jump = c.w;
                     }
@@ -871,21 +914,21 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
     }
 }
 
-template <int T, int VM>
+template <int T, int VM, class LG>
 cudaError_t launch_t(cudaStream_t s, const SearchParams& p, int blocks, int bt, bool persistent,
                      int req_base, int bm_words) {
     // the dynamic shared-memory limit was raised when the search state was
     // sized (no attribute calls here: this may run under stream capture)
     const size_t smem = smem_bytes(p.C, bt, bm_words, T, VM, p.queues != nullptr, p.full_pad != 0);
     if (blocks <= 0) return cudaSuccess;
-    k_corridor_search<T, VM><<<blocks, bt, smem, s>>>(p, persistent ? 1 : 0, req_base, bm_words);
+    k_corridor_search<T, VM, LG><<<blocks, bt, smem, s>>>(p, persistent ? 1 : 0, req_base, bm_words);
     return cudaGetLastError();
 }
 
 // the kernel's dynamic shared-memory limit (only ever raised, as for search.cu's kernel)
 std::mutex g_smem_attr_mu;
 
-template <int T, int VM>
+template <int T, int VM, class LG>
 bool raise_smem_limit(int smem) {
     static int limit[64] = {};
     int device = 0;
@@ -895,7 +938,7 @@ bool raise_smem_limit(int smem) {
     }
     std::lock_guard<std::mutex> lock(g_smem_attr_mu);
     if (smem > limit[device & 63]) {
-        if (cudaFuncSetAttribute(k_corridor_search<T, VM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+        if (cudaFuncSetAttribute(k_corridor_search<T, VM, LG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
             cudaSuccess) {
             cudaGetLastError();
             return false;
@@ -905,28 +948,28 @@ bool raise_smem_limit(int smem) {
     return true;
 }
 
-template <int T, int VM>
+template <int T, int VM, class LG>
 int occupancy_t(int C, int bt, int bm_words, bool queues_global, bool full_pad) {
     if (bt > 256) return 0;  // the kernel's launch bounds
     const size_t smem = smem_bytes(C, bt, bm_words, T, VM, queues_global, full_pad);
-    if (smem > 227 * 1024 || !raise_smem_limit<T, VM>((int)smem)) return 0;
+    if (smem > 227 * 1024 || !raise_smem_limit<T, VM, LG>((int)smem)) return 0;
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_corridor_search<T, VM>, bt, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_corridor_search<T, VM, LG>, bt, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     return nb;
 }
 
-template <int VM>
+template <int VM, class LG>
 cudaError_t launch_v(cudaStream_t s, const SearchParams& p, int blocks, int bt, bool persistent,
                      int req_base, int bm_words) {
     switch (p.T) {
-        case 2: return launch_t<2, VM>(s, p, blocks, bt, persistent, req_base, bm_words);
-        case 4: return launch_t<4, VM>(s, p, blocks, bt, persistent, req_base, bm_words);
-        case 8: return launch_t<8, VM>(s, p, blocks, bt, persistent, req_base, bm_words);
-        case 16: return launch_t<16, VM>(s, p, blocks, bt, persistent, req_base, bm_words);
-        case 32: return launch_t<32, VM>(s, p, blocks, bt, persistent, req_base, bm_words);
+        case 2: return launch_t<2, VM, LG>(s, p, blocks, bt, persistent, req_base, bm_words);
+        case 4: return launch_t<4, VM, LG>(s, p, blocks, bt, persistent, req_base, bm_words);
+        case 8: return launch_t<8, VM, LG>(s, p, blocks, bt, persistent, req_base, bm_words);
+        case 16: return launch_t<16, VM, LG>(s, p, blocks, bt, persistent, req_base, bm_words);
+        case 32: return launch_t<32, VM, LG>(s, p, blocks, bt, persistent, req_base, bm_words);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -934,11 +977,11 @@ cudaError_t launch_v(cudaStream_t s, const SearchParams& p, int blocks, int bt, 
 template <int VM>
 int occupancy_v(int T, int C, int bt, int bm_words, bool qg, bool full_pad) {
     switch (T) {
-        case 2: return occupancy_t<2, VM>(C, bt, bm_words, qg, full_pad);
-        case 4: return occupancy_t<4, VM>(C, bt, bm_words, qg, full_pad);
-        case 8: return occupancy_t<8, VM>(C, bt, bm_words, qg, full_pad);
-        case 16: return occupancy_t<16, VM>(C, bt, bm_words, qg, full_pad);
-        case 32: return occupancy_t<32, VM>(C, bt, bm_words, qg, full_pad);
+        case 2: return occupancy_t<2, VM, WideLog>(C, bt, bm_words, qg, full_pad);
+        case 4: return occupancy_t<4, VM, WideLog>(C, bt, bm_words, qg, full_pad);
+        case 8: return occupancy_t<8, VM, WideLog>(C, bt, bm_words, qg, full_pad);
+        case 16: return occupancy_t<16, VM, WideLog>(C, bt, bm_words, qg, full_pad);
+        case 32: return occupancy_t<32, VM, WideLog>(C, bt, bm_words, qg, full_pad);
         default: return 0;
     }
 }
@@ -951,11 +994,11 @@ size_t corridor_smem_bytes(int C, int bt, int bm_words, int T, int vm) {
 
 bool corridor_full_smem(int T) {
     switch (T) {
-        case 2: return raise_smem_limit<2, 1>(227 * 1024);
-        case 4: return raise_smem_limit<4, 1>(227 * 1024);
-        case 8: return raise_smem_limit<8, 1>(227 * 1024);
-        case 16: return raise_smem_limit<16, 1>(227 * 1024);
-        case 32: return raise_smem_limit<32, 1>(227 * 1024);
+        case 2: return raise_smem_limit<2, 1, WideLog>(227 * 1024) && raise_smem_limit<2, 1, PackedLog>(227 * 1024);
+        case 4: return raise_smem_limit<4, 1, WideLog>(227 * 1024) && raise_smem_limit<4, 1, PackedLog>(227 * 1024);
+        case 8: return raise_smem_limit<8, 1, WideLog>(227 * 1024) && raise_smem_limit<8, 1, PackedLog>(227 * 1024);
+        case 16: return raise_smem_limit<16, 1, WideLog>(227 * 1024) && raise_smem_limit<16, 1, PackedLog>(227 * 1024);
+        case 32: return raise_smem_limit<32, 1, WideLog>(227 * 1024) && raise_smem_limit<32, 1, PackedLog>(227 * 1024);
         default: return false;
     }
 }
@@ -973,8 +1016,10 @@ int corridor_max_blocks_per_sm(int T, int C, int bt, int vm, int bm_words, bool 
 cudaError_t launch_corridor_search(cudaStream_t s, const SearchParams& p, int blocks, int bt, bool persistent,
                                    int req_base, int vm, int bm_words) {
     switch (vm) {
-        case 1: return launch_v<1>(s, p, blocks, bt, persistent, req_base, bm_words);
-        case 4: return launch_v<4>(s, p, blocks, bt, persistent, req_base, bm_words);
+        case 1:
+            return p.log_packed ? launch_v<1, PackedLog>(s, p, blocks, bt, persistent, req_base, bm_words)
+                                : launch_v<1, WideLog>(s, p, blocks, bt, persistent, req_base, bm_words);
+        case 4: return p.log_packed ? cudaErrorInvalidValue : launch_v<4, WideLog>(s, p, blocks, bt, persistent, req_base, bm_words);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -52,10 +52,10 @@ constexpr size_t kWorkOff = 0, kQueryOff = 8, kErrOff = 16, kStatsOff = 64;
 
 // Query stamps of the record form start here.  The log form leaves edge rows,
 // centroids and log entries in the same array; the upper word of a stamp, read
-// as any of those, would be an index or a depth of two billion or a signalling
-// NaN, which no arithmetic makes: what the one form leaves is never live to the
-// other.
-constexpr unsigned long long kFirstStamp = 0x7f900000ull << 32;
+// as any of those, would be an index or a depth far below zero, a packed entry's
+// second word with its free top bit set, or a signalling NaN, which no arithmetic
+// makes: what the one form leaves is never live to the other.
+constexpr unsigned long long kFirstStamp = 0xff900000ull << 32;
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
@@ -359,10 +359,10 @@ __global__ void __launch_bounds__(32) k_search_noalloc(NoAllocArgs a) {
 // ---- the log form: the search of corridor.cu in the same scratch array ----
 // Each call first lays out the navmesh as that kernel reads it (edge rows, third
 // candidates, centroids: 152 bytes per triangle), then searches with claim logs
-// of 16 bytes per triangle and slot and the visited bitmaps in shared memory.
-// On the 17,406-triangle maze that is 1.8 times the slots of the record form
-// (the slots that fit the array bound large navmeshes: 218 searches at a time
-// there), and shorter rounds: 2,048 queries at T=8, C=32 took 34.4 ms, now 9.1;
+// of 16 bytes per triangle and slot (8 up to kPackedLogNodes triangles) and the
+// visited bitmaps in shared memory.  The slots that fit the array bound large
+// navmeshes: on the 17,406-triangle maze 460 searches at a time, 120 in the record
+// form, and rounds are shorter: 2,048 queries at T=8, C=32 took 34.4 ms, now 5.6 (8.2 with 16-byte entries);
 // 37 on the 104,958-triangle maze at T=32, C=16 21.0, now 4.6; 2,048 between
 // rectangles (1,313 triangles) 0.148, now 0.118.  The record form stays for
 // navmeshes whose rows leave too few slots.
@@ -416,7 +416,8 @@ struct LogLayout {
     EdgeRow* rows;
     EdgeHalf* third;
     float2* cen;
-    int4* logs;
+    void* logs;
+    bool packed;
     long long slots;  // 0: does not fit
 };
 LogLayout log_layout(unsigned char* scratch, int n) {
@@ -424,8 +425,9 @@ LogLayout log_layout(unsigned char* scratch, int n) {
     const size_t rows = up(kHeaderBytes), third = up(rows + sizeof(EdgeRow) * 4 * (size_t)n),
                  cen = up(third + sizeof(EdgeHalf) * (size_t)n), logs = up(cen + sizeof(float2) * (size_t)n);
     LogLayout l{reinterpret_cast<EdgeRow*>(scratch + rows), reinterpret_cast<EdgeHalf*>(scratch + third),
-                reinterpret_cast<float2*>(scratch + cen), reinterpret_cast<int4*>(scratch + logs), 0};
-    if (logs < kScratchBytes) l.slots = (long long)((kScratchBytes - logs) / (sizeof(int4) * (size_t)n));
+                reinterpret_cast<float2*>(scratch + cen), scratch + logs, n <= kPackedLogNodes, 0};
+    if (logs < kScratchBytes)
+        l.slots = (long long)((kScratchBytes - logs) / ((l.packed ? sizeof(uint2) : sizeof(int4)) * (size_t)n));
     return l;
 }
 
@@ -595,6 +597,7 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
         p.C = C;
         p.K = heuristic_k;
         p.log = lay.logs;
+        p.log_packed = lay.packed;
         p.slots = blocks_log;
         p.work_ctr = reinterpret_cast<int*>(ds->scratch + kWorkOff);
         p.max_rounds = a.max_rounds;

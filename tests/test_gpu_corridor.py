@@ -109,6 +109,37 @@ def test_noalloc_log_form(lib, oracle_mod, T, Cap):
             assert np.array_equal(gp[i, :gl[i]], op[i, :gl[i]])
 
 
+@pytest.mark.parametrize("n", [2**15, 2**15 + 1])
+def test_noalloc_log_entry_sizes(lib, oracle_mod, n):
+    # the largest navmesh with 8-byte log entries and the smallest with 16: ids,
+    # log places and depths (searches of a triangle nobody lists run to the
+    # strip's other end) up to the ends of their fields
+    import ctypes as C
+    import torch
+    T, Cap, q = 8, 32, 40
+    nodes = strip_map(n, 2, seed=13)
+    nb = nodes["NeibsIdx"]
+    nb[nb == n - 2] = n - 1
+    nb[n - 2] = -1
+    rng = np.random.default_rng(14)
+    s, t = (rng.integers(0, n, q).astype(np.int32) for _ in range(2))
+    s[:4], t[:4] = [0, 1, n - 1, n - 1], [n - 2, n - 1, 0, n - 2]
+    of, ol, op, _ = oracle_mod.OMap(nodes).search_batch(s, t, T, Cap)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    d_nodes, d_s, d_t = dev(nodes.view(np.uint8)), dev(s), dev(t)
+    f, l = (torch.full((q,), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+    p = torch.full((q, n), -7, dtype=torch.int32, device="cuda")
+    rc = lib.gmapf_search_batch_noalloc(d_nodes.data_ptr(), n, d_s.data_ptr(), d_t.data_ptr(), q, T, Cap,
+                                        C.c_float(1.0), 0, f.data_ptr(), l.data_ptr(), p.data_ptr(), n,
+                                        C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert rc == 0
+    gf, gl, gp = f.cpu().numpy(), l.cpu().numpy(), p.cpu().numpy()
+    assert np.array_equal(gf, of) and np.array_equal(gl, ol) and gl.max() > n // 4
+    for i in np.nonzero(gf)[0]:
+        assert np.array_equal(gp[i, :gl[i]], op[i, :gl[i]])
+
+
 def test_scene_batch_and_serving_on_corridors(oracle_mod):
     # two winding corridors stepped as one batch, then one of them served: the
     # corridor kernel with global ids, and on the serving streams

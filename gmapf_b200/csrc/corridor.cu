@@ -46,39 +46,59 @@ constexpr int kJumpDepth = 32;
 
 // An entry as it is: one 16-byte access.
 struct WideLog {
-    using Entry = int4;
     int4* p;
-    __device__ __forceinline__ int4 get(int i) const { return __ldcg(p + i); }
-    __device__ __forceinline__ int2 claim(int i) const { return __ldcg(reinterpret_cast<const int2*>(p + i)); }
+    __device__ __forceinline__ WideLog(const SearchParams& a, int slot)
+        : p(static_cast<int4*>(a.log) + (size_t)(a.slot_base + slot) * a.n) {}
+    __device__ __forceinline__ int2 hop(int i) const {  // {directed edge, parent's entry}
+        const int4 q = __ldcg(p + i);
+        return make_int2(q.x, q.z);
+    }
     __device__ __forceinline__ int edge(int i) const { return __ldcg(&p[i].x); }
-    __device__ __forceinline__ int key(int i) const { return __ldcg(&p[i].y); }
+    __device__ __forceinline__ int2 edge_jump(int i) const {
+        const int4 q = __ldcg(p + i);
+        return make_int2(q.x, q.w);
+    }
     __device__ __forceinline__ int jump(int i) const { return __ldcg(&p[i].w); }
-    __device__ __forceinline__ void put(int i, int4 q) const { __stcg(p + i, q); }
+    __device__ __forceinline__ int depth(int i) const { return __ldcg(&p[i].y) >> 1; }
+    __device__ __forceinline__ void put(int i, int e, int gd, int parent, int jump) const {
+        __stcg(p + i, make_int4(e, gd, parent, jump));
+    }
 };
 
-// In 8 bytes, for maps of at most kPackedLogNodes triangles: edge 17 bits, G<<1|dir
-// 16 (a depth is below the claims), parent + 1 and jump + 1 15 each (an ancestor is
-// an earlier claim).  Twice the searches in a fixed scratch array (searches without
-// allocation).  Where memory is not the limit the wide entry costs fewer
-// instructions: 64x64-cell maze, placement 1, 16,384 searches at T=4 14.5 against
-// 14.9 ms, T=8 6.9 against 7.0, 37 searches 0.575 against 0.603; at T=32 the packed
-// one is 0-6% faster, within what its runs differ by.
+// In 6 bytes, for maps of at most kPackedLogNodes triangles: a word of the edge (17
+// bits) and parent + 1 (15; an ancestor is an earlier claim), a half word of
+// jump + 1.  The depth is not kept: it follows from the jump chain's length.
+// 2.7 times the searches in a fixed scratch array (searches without allocation).
+// Where memory is not the limit the wide entry costs fewer instructions: 64x64-cell
+// maze, placement 1, packed in 8 bytes, 16,384 searches at T=4 14.5 against 14.9
+// ms, T=8 6.9 against 7.0, 37 searches 0.575 against 0.603; at T=32 the packed one
+// was 0-6% faster, within what its runs differ by.
 struct PackedLog {
-    using Entry = uint2;
-    uint2* p;
-    static __device__ __forceinline__ int4 unpack(uint2 v) {
-        return make_int4((int)(v.x & 0x1ffffu), (int)(v.y & 0xffffu), (int)(v.x >> 17) - 1, (int)(v.y >> 16) - 1);
+    unsigned* p;         // slots x n words, then slots x n half words
+    unsigned short* pj;
+    __device__ __forceinline__ PackedLog(const SearchParams& a, int slot)
+        : p(static_cast<unsigned*>(a.log) + (size_t)slot * a.n),
+          pj(reinterpret_cast<unsigned short*>(static_cast<unsigned*>(a.log) + (size_t)a.slots * a.n) +
+             (size_t)slot * a.n) {}
+    __device__ __forceinline__ int2 hop(int i) const {
+        const unsigned v = __ldcg(p + i);
+        return make_int2((int)(v & 0x1ffffu), (int)(v >> 17) - 1);
     }
-    __device__ __forceinline__ int4 get(int i) const { return unpack(__ldcg(p + i)); }
-    __device__ __forceinline__ int2 claim(int i) const {
-        const int4 q = get(i);
-        return make_int2(q.x, q.y);
+    __device__ __forceinline__ int edge(int i) const { return (int)(__ldcg(p + i) & 0x1ffffu); }
+    __device__ __forceinline__ int jump(int i) const { return (int)__ldcg(pj + i) - 1; }
+    __device__ __forceinline__ int2 edge_jump(int i) const { return make_int2(edge(i), jump(i)); }
+    __device__ __forceinline__ int depth(int i) const { return depth_of(p, pj, i); }
+    static __device__ __noinline__ int depth_of(const unsigned* p, const unsigned short* pj, int i) {
+        const int first = (int)__ldcg(pj + i) - 1;  // the nearest ancestor at a multiple of kJumpDepth
+        if (first < 0) return 0;                    // a root
+        int d = 0;
+        for (int x = i; x != first && x >= 0 && d <= kJumpDepth; x = (int)(__ldcg(p + x) >> 17) - 1) d++;
+        for (int y = first; (y = (int)__ldcg(pj + y) - 1) >= 0;) d += kJumpDepth;  // (ever earlier entries)
+        return d;
     }
-    __device__ __forceinline__ int edge(int i) const { return get(i).x; }
-    __device__ __forceinline__ int key(int i) const { return get(i).y; }
-    __device__ __forceinline__ int jump(int i) const { return get(i).w; }
-    __device__ __forceinline__ void put(int i, int4 q) const {
-        __stcg(p + i, make_uint2((unsigned)q.x | (unsigned)(q.z + 1) << 17, (unsigned)q.y | (unsigned)(q.w + 1) << 16));
+    __device__ __forceinline__ void put(int i, int e, int, int parent, int jump) const {
+        __stcg(p + i, (unsigned)e | (unsigned)(parent + 1) << 17);
+        __stcg(pj + i, (unsigned short)(jump + 1));
     }
 };
 static_assert(kPackedLogNodes <= 1 << 15, "PackedLog: an edge has 17 bits, an entry 15");
@@ -135,33 +155,26 @@ __host__ __device__ __forceinline__ size_t corridor_frontier_words(int T) {
     return (size_t)4 * 3 * T + kSeenWords + 8 * corridor_staged_rows(T) + ((3 * T + 15) / 16) * 4;
 }
 
-// The log entry and G<<1|dir of node n (claimed by this search), newest first;
-// -1 if none.  The other side's claim of the meeting node can be old (a queue
+// The log entry of node n (claimed by this search), newest first; -1 if none.  The other side's claim of the meeting node can be old (a queue
 // dropped it): on the 160x160 maze 9-15 thousand claims back on average.
 template <class LG>
-__device__ __noinline__ int2 find_claim(LG log, int claims, int n, int lane) {
+__device__ __noinline__ int find_claim(LG log, int claims, int n, int lane) {
     constexpr int U = 8;  // 256 entries per step, all reads in flight
     for (int top = claims; top > 0; top -= 32 * U) {
-        int2 q[U];
+        int q[U];
 #pragma unroll
         for (int j = 0; j < U; j++) {
             const int i = top - 1 - (j * 32 + lane);
-            q[j] = i >= 0 ? log.claim(i) : make_int2(-1, 0);
+            q[j] = i >= 0 ? log.edge(i) : -1;
         }
-        int hit = -1, gd = 0;
+        int hit = -1;
 #pragma unroll
         for (int j = 0; j < U; j++)
-            if ((q[j].x >> 2) == n) {
-                hit = top - 1 - (j * 32 + lane);
-                gd = q[j].y;
-            }
+            if ((q[j] >> 2) == n) hit = top - 1 - (j * 32 + lane);
         const unsigned m = __ballot_sync(kFull, hit >= 0);
-        if (m) {
-            const int l = __ffs(m) - 1;
-            return make_int2(__shfl_sync(kFull, hit, l), __shfl_sync(kFull, gd, l));
-        }
+        if (m) return __shfl_sync(kFull, hit, __ffs(m) - 1);
     }
-    return make_int2(-1, 0);
+    return -1;
 }
 
 // Path walk of one warp.  Lanes 0 and 1 follow each side's jump chain from the
@@ -179,8 +192,8 @@ __device__ __forceinline__ void walk_path(LG log, int claims, int2* buf, int cap
         __syncwarp();
 #pragma unroll 4
         for (int i = lane; i < claims; i += 32) {
-            const int4 q = log.get(i);
-            buf[i] = make_int2(q.x >> 2, q.z);
+            const int2 q = log.hop(i);
+            buf[i] = make_int2(q.x >> 2, q.y);
         }
         __syncwarp();
         if (lane < 2) {
@@ -252,7 +265,7 @@ __device__ __forceinline__ void walk_path(LG log, int claims, int2* buf, int cap
         bool more = true;
         while (more) {
             more = false;
-            int4 q[W];
+            int2 q[W];
 #pragma unroll
             for (int j = 0; j < W; j++) {
                 if (d[j] < b[j]) continue;
@@ -262,13 +275,13 @@ __device__ __forceinline__ void walk_path(LG log, int claims, int2* buf, int cap
                     b[j] = 0;
                     continue;
                 }
-                q[j] = log.get(x[j]);
+                q[j] = log.hop(x[j]);
             }
 #pragma unroll
             for (int j = 0; j < W; j++) {
                 if (d[j] < b[j]) continue;
                 out[path_pos(sd[j], d[j], gS, gT)] = q[j].x >> 2;
-                x[j] = q[j].z;
+                x[j] = q[j].y;
                 d[j]--;
                 more = true;
             }
@@ -341,7 +354,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
 
     if (slot >= p.slots) return;  // whole warps
     if (VM == 4) bm = p.gbm + (size_t)(p.slot_base + slot) * bm_words;
-    const LG log{static_cast<typename LG::Entry*>(p.log) + (size_t)(p.slot_base + slot) * n_nodes};
+    const LG log(p, slot);
     const unsigned lt_mask = (1u << lane) - 1u;
 
     for (int iter = 0;; iter++) {
@@ -434,7 +447,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
             e = (node << 2) | 3;
             at = k;
             if (lane < 2) {
-                log.put(lane, make_int4(e, gd, -1, -1));
+                log.put(lane, e, gd, -1, -1);
                 bm_set<SMEMV>(bm, node, gd);
             }
         }
@@ -479,28 +492,22 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
             auto write_claim = [&](int i, int en, float cx, float cy) {
                 const float F = GM_FADD(gf, GM_FMUL(dist_sqr(cx, cy, farx, fary), K));
                 fr[i] = make_int4(__float_as_int(F), ngd, en, cjump);
-                log.put(claims + i, make_int4(en, ngd, at, cjump));
+                log.put(claims + i, en, ngd, at, cjump);
             };
 
             // the search's end: node mn, log entry `other` (-1: look for it), met from log entry mat with key mgd
             auto finish = [&](int mat, int mgd, int mn, int other) {
-                int ogd;
-                if (other >= 0) {
-                    ogd = log.key(other);
-                } else {
-                    const int2 f = find_claim(log, claims, mn, lane);
-                    other = f.x;
-                    ogd = f.y;
-                }
+                if (other < 0) other = find_claim(log, claims, mn, lane);
                 if (other < 0) {
                     if (lane == 0) atomicOr(p.err, ERR_BOUNDS);
                     return;
                 }
+                const int og = log.depth(other);
                 const bool from_start = mgd & 1;  // PathFinder.h:226-227
                 mS = from_start ? mat : other;
-                gS = (from_start ? mgd : ogd) >> 1;
+                gS = from_start ? mgd >> 1 : og;
                 mT = from_start ? other : mat;
-                gT = (from_start ? ogd : mgd) >> 1;
+                gT = from_start ? og : mgd >> 1;
                 found = 1;
             };
             // A candidate whose node nobody claimed is this lane's claim (g) unless
@@ -792,9 +799,9 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
                         top.F = __int_as_float(w.x);
                         top.gd = w.y;
                         top.at = ring.id()[k];
-                        const int4 c = log.get(top.at);
+                        const int2 c = log.edge_jump(top.at);
                         top.e = c.x;
-                        top.jump = c.w;
+                        top.jump = c.y;
                     }
                 }
             }

@@ -52,9 +52,9 @@ constexpr size_t kWorkOff = 0, kQueryOff = 8, kErrOff = 16, kStatsOff = 64;
 
 // Query stamps of the record form start here.  The log form leaves edge rows,
 // centroids and log entries in the same array; the upper word of a stamp, read
-// as any of those, would be an index or a depth far below zero, a packed entry's
-// second word with its free top bit set, or a signalling NaN, which no arithmetic
-// makes: what the one form leaves is never live to the other.
+// as any of those, would be an index or a depth far below zero, a packed log
+// entry beyond kPackedLogNodes, or a signalling NaN, which no arithmetic makes: what
+// the one form leaves is never live to the other.
 constexpr unsigned long long kFirstStamp = 0xff900000ull << 32;
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
@@ -359,13 +359,13 @@ __global__ void __launch_bounds__(32) k_search_noalloc(NoAllocArgs a) {
 // ---- the log form: the search of corridor.cu in the same scratch array ----
 // Each call first lays out the navmesh as that kernel reads it (edge rows, third
 // candidates, centroids: 152 bytes per triangle), then searches with claim logs
-// of 16 bytes per triangle and slot (8 up to kPackedLogNodes triangles) and the
+// of 16 bytes per triangle and slot (6 up to kPackedLogNodes triangles) and the
 // visited bitmaps in shared memory.  The slots that fit the array bound large
-// navmeshes: on the 17,406-triangle maze 460 searches at a time, 120 in the record
-// form, and rounds are shorter: 2,048 queries at T=8, C=32 took 34.4 ms, now 5.6 (8.2 with 16-byte entries);
-// 37 on the 104,958-triangle maze at T=32, C=16 21.0, now 4.6; 2,048 between
-// rectangles (1,313 triangles) 0.148, now 0.118.  The record form stays for
-// navmeshes whose rows leave too few slots.
+// navmeshes: on the 17,406-triangle maze 617 searches at a time, 120 in the record
+// form, and rounds are shorter: 2,048 queries at T=8, C=32 took 34.4 ms, now 4.7 (8.2
+// with 16-byte entries, 5.6 with 8); 37 on the 104,958-triangle maze at T=32, C=16
+// 21.0, now 4.6; 2,048 between rectangles (1,313 triangles) 0.148, now 0.118.  The
+// record form stays for navmeshes whose rows leave too few slots.
 
 // search.cu's SearchRow rules on caller-provided records: the neighbours up to
 // the first -1; ids outside the navmesh keep their slot but are no candidates
@@ -427,7 +427,7 @@ LogLayout log_layout(unsigned char* scratch, int n) {
     LogLayout l{reinterpret_cast<EdgeRow*>(scratch + rows), reinterpret_cast<EdgeHalf*>(scratch + third),
                 reinterpret_cast<float2*>(scratch + cen), scratch + logs, n <= kPackedLogNodes, 0};
     if (logs < kScratchBytes)
-        l.slots = (long long)((kScratchBytes - logs) / ((l.packed ? sizeof(uint2) : sizeof(int4)) * (size_t)n));
+        l.slots = (long long)((kScratchBytes - logs) / ((l.packed ? 6 : sizeof(int4)) * (size_t)n));
     return l;
 }
 

@@ -109,9 +109,9 @@ def test_noalloc_log_form(lib, oracle_mod, T, Cap):
             assert np.array_equal(gp[i, :gl[i]], op[i, :gl[i]])
 
 
-@pytest.mark.parametrize("n", [2**15, 2**15 + 1])
+@pytest.mark.parametrize("n", [0x7fc0, 0x7fc1])
 def test_noalloc_log_entry_sizes(lib, oracle_mod, n):
-    # the largest navmesh with 8-byte log entries and the smallest with 16: ids,
+    # the largest navmesh with 6-byte log entries and the smallest with 16: ids,
     # log places and depths (searches of a triangle nobody lists run to the
     # strip's other end) up to the ends of their fields
     import ctypes as C

@@ -65,10 +65,45 @@ struct WideLog {
     }
 };
 
+// The depth of an entry that does not keep it follows from the jump chain's length.
+template <class LG>
+__device__ __noinline__ int depth_by_jumps(LG log, int i) {
+    const int first = log.jump(i);  // the nearest ancestor at a multiple of kJumpDepth
+    if (first < 0) return 0;        // a root
+    int d = 0;
+    for (int x = i; x != first && x >= 0 && d <= kJumpDepth; x = log.hop(x).y) d++;
+    for (int y = first; (y = log.jump(y)) >= 0;) d += kJumpDepth;  // (ever earlier entries)
+    return d;
+}
+
+// In 8 bytes, for maps of at most 2^20 triangles: edge 22 bits, parent + 1 and
+// jump + 1 20 bits each (an ancestor is an earlier claim).
+struct HalfLog {
+    unsigned long long* p;
+    __device__ __forceinline__ HalfLog(const SearchParams& a, int slot)
+        : p(static_cast<unsigned long long*>(a.log) + (size_t)slot * a.n) {}
+    __device__ __forceinline__ unsigned long long at(int i) const { return __ldcg(p + i); }
+    __device__ __forceinline__ int2 hop(int i) const {
+        const unsigned long long v = at(i);
+        return make_int2((int)(v & 0x3fffffu), (int)((v >> 22) & 0xfffffu) - 1);
+    }
+    __device__ __forceinline__ int edge(int i) const { return (int)(at(i) & 0x3fffffu); }
+    __device__ __forceinline__ int jump(int i) const { return (int)(at(i) >> 42) - 1; }
+    __device__ __forceinline__ int2 edge_jump(int i) const {
+        const unsigned long long v = at(i);
+        return make_int2((int)(v & 0x3fffffu), (int)(v >> 42) - 1);
+    }
+    __device__ __forceinline__ int depth(int i) const { return depth_by_jumps(*this, i); }
+    __device__ __forceinline__ void put(int i, int e, int, int parent, int jump) const {
+        __stcg(p + i, (unsigned long long)(unsigned)e | (unsigned long long)(unsigned)(parent + 1) << 22 |
+                          (unsigned long long)(unsigned)(jump + 1) << 42);
+    }
+};
+static_assert(kHalfLogNodes <= 1 << 20, "HalfLog: an edge has 22 bits, an entry 20");
+
 // In 6 bytes, for maps of at most kPackedLogNodes triangles: a word of the edge (17
 // bits) and parent + 1 (15; an ancestor is an earlier claim), a half word of
-// jump + 1.  The depth is not kept: it follows from the jump chain's length.
-// 2.7 times the searches in a fixed scratch array (searches without allocation).
+// jump + 1.  2.7 times the searches of WideLog in a fixed scratch array (searches without allocation).
 // Where memory is not the limit the wide entry costs fewer instructions: 64x64-cell
 // maze, placement 1, packed in 8 bytes, 16,384 searches at T=4 14.5 against 14.9
 // ms, T=8 6.9 against 7.0, 37 searches 0.575 against 0.603; at T=32 the packed one
@@ -87,15 +122,7 @@ struct PackedLog {
     __device__ __forceinline__ int edge(int i) const { return (int)(__ldcg(p + i) & 0x1ffffu); }
     __device__ __forceinline__ int jump(int i) const { return (int)__ldcg(pj + i) - 1; }
     __device__ __forceinline__ int2 edge_jump(int i) const { return make_int2(edge(i), jump(i)); }
-    __device__ __forceinline__ int depth(int i) const { return depth_of(p, pj, i); }
-    static __device__ __noinline__ int depth_of(const unsigned* p, const unsigned short* pj, int i) {
-        const int first = (int)__ldcg(pj + i) - 1;  // the nearest ancestor at a multiple of kJumpDepth
-        if (first < 0) return 0;                    // a root
-        int d = 0;
-        for (int x = i; x != first && x >= 0 && d <= kJumpDepth; x = (int)(__ldcg(p + x) >> 17) - 1) d++;
-        for (int y = first; (y = (int)__ldcg(pj + y) - 1) >= 0;) d += kJumpDepth;  // (ever earlier entries)
-        return d;
-    }
+    __device__ __forceinline__ int depth(int i) const { return depth_by_jumps(*this, i); }
     __device__ __forceinline__ void put(int i, int e, int, int parent, int jump) const {
         __stcg(p + i, (unsigned)e | (unsigned)(parent + 1) << 17);
         __stcg(pj + i, (unsigned short)(jump + 1));
@@ -999,13 +1026,20 @@ size_t corridor_smem_bytes(int C, int bt, int bm_words, int T, int vm) {
     return smem_bytes(C, bt, bm_words, T, vm, false, false);
 }
 
+template <int T>
+static bool full_smem_t() {
+    constexpr int kAll = 227 * 1024;
+    return raise_smem_limit<T, 1, WideLog>(kAll) && raise_smem_limit<T, 1, HalfLog>(kAll) &&
+           raise_smem_limit<T, 1, PackedLog>(kAll);
+}
+
 bool corridor_full_smem(int T) {
     switch (T) {
-        case 2: return raise_smem_limit<2, 1, WideLog>(227 * 1024) && raise_smem_limit<2, 1, PackedLog>(227 * 1024);
-        case 4: return raise_smem_limit<4, 1, WideLog>(227 * 1024) && raise_smem_limit<4, 1, PackedLog>(227 * 1024);
-        case 8: return raise_smem_limit<8, 1, WideLog>(227 * 1024) && raise_smem_limit<8, 1, PackedLog>(227 * 1024);
-        case 16: return raise_smem_limit<16, 1, WideLog>(227 * 1024) && raise_smem_limit<16, 1, PackedLog>(227 * 1024);
-        case 32: return raise_smem_limit<32, 1, WideLog>(227 * 1024) && raise_smem_limit<32, 1, PackedLog>(227 * 1024);
+        case 2: return full_smem_t<2>();
+        case 4: return full_smem_t<4>();
+        case 8: return full_smem_t<8>();
+        case 16: return full_smem_t<16>();
+        case 32: return full_smem_t<32>();
         default: return false;
     }
 }
@@ -1024,9 +1058,12 @@ cudaError_t launch_corridor_search(cudaStream_t s, const SearchParams& p, int bl
                                    int req_base, int vm, int bm_words) {
     switch (vm) {
         case 1:
-            return p.log_packed ? launch_v<1, PackedLog>(s, p, blocks, bt, persistent, req_base, bm_words)
-                                : launch_v<1, WideLog>(s, p, blocks, bt, persistent, req_base, bm_words);
-        case 4: return p.log_packed ? cudaErrorInvalidValue : launch_v<4, WideLog>(s, p, blocks, bt, persistent, req_base, bm_words);
+            switch (p.log_bytes) {
+                case 6: return launch_v<1, PackedLog>(s, p, blocks, bt, persistent, req_base, bm_words);
+                case 8: return launch_v<1, HalfLog>(s, p, blocks, bt, persistent, req_base, bm_words);
+                default: return launch_v<1, WideLog>(s, p, blocks, bt, persistent, req_base, bm_words);
+            }
+        case 4: return launch_v<4, WideLog>(s, p, blocks, bt, persistent, req_base, bm_words);
         default: return cudaErrorInvalidValue;
     }
 }

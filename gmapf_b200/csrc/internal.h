@@ -83,7 +83,7 @@ struct SearchParams {
     Rec* rec;                // slots * n
     unsigned* epoch;         // per slot
     void* log;               // corridor maps, instead of rec: slots * n, the claims of a slot's search in order
-    int log_packed;          // its entries take 6 bytes (n <= kPackedLogNodes), not 16
+    int log_bytes;           // placement 1: its entries take 6 bytes (n <= kPackedLogNodes) or 8 (kHalfLogNodes), 0: 16
     int* queues;             // corridor maps: slots x corridor_queue_bytes, or null (queues in shared memory)
     int slots;
     unsigned* gbm;           // visited mode 3: bm_words 32-bit words per slot, global
@@ -241,7 +241,7 @@ int corridor_max_blocks_per_sm(int T, int C, int block_threads, int vm, int bm_w
 size_t corridor_queue_bytes(int C, int T);
 // (an edge in 17 bits, an entry in 15; words of packed logs stay below 0xff800000:
 // see kFirstStamp in noalloc.cu)
-constexpr int kPackedLogNodes = 0x7fc0;
+constexpr int kPackedLogNodes = 0x7fc0, kHalfLogNodes = 1 << 20;
 size_t corridor_smem_bytes(int C, int block_threads, int bm_words, int T, int vm);
 // lets visited placement 1 use all the shared memory of an SM on the current
 // device (so that later launches need no attribute call); false: a CUDA error

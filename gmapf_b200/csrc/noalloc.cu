@@ -359,12 +359,13 @@ __global__ void __launch_bounds__(32) k_search_noalloc(NoAllocArgs a) {
 // ---- the log form: the search of corridor.cu in the same scratch array ----
 // Each call first lays out the navmesh as that kernel reads it (edge rows, third
 // candidates, centroids: 152 bytes per triangle), then searches with claim logs
-// of 16 bytes per triangle and slot (6 up to kPackedLogNodes triangles) and the
+// of 6 bytes per triangle and slot (8 above kPackedLogNodes triangles) and the
 // visited bitmaps in shared memory.  The slots that fit the array bound large
 // navmeshes: on the 17,406-triangle maze 617 searches at a time, 120 in the record
 // form, and rounds are shorter: 2,048 queries at T=8, C=32 took 34.4 ms, now 4.7 (8.2
-// with 16-byte entries, 5.6 with 8); 37 on the 104,958-triangle maze at T=32, C=16
-// 21.0, now 4.6; 2,048 between rectangles (1,313 triangles) 0.148, now 0.118.  The
+// with 16-byte entries, 5.6 with 8).  On the 104,958-triangle maze 2,048 queries take
+// 145 ms (270 with 16-byte entries), 37 at T=32, C=16 took 21.0, now 2.9; 2,048
+// between rectangles (1,313 triangles) 0.148, now 0.118 (its own log is no limit).  The
 // record form stays for navmeshes whose rows leave too few slots.
 
 // search.cu's SearchRow rules on caller-provided records: the neighbours up to
@@ -417,7 +418,7 @@ struct LogLayout {
     EdgeHalf* third;
     float2* cen;
     void* logs;
-    bool packed;
+    int entry;        // bytes of a log entry
     long long slots;  // 0: does not fit
 };
 LogLayout log_layout(unsigned char* scratch, int n) {
@@ -425,11 +426,12 @@ LogLayout log_layout(unsigned char* scratch, int n) {
     const size_t rows = up(kHeaderBytes), third = up(rows + sizeof(EdgeRow) * 4 * (size_t)n),
                  cen = up(third + sizeof(EdgeHalf) * (size_t)n), logs = up(cen + sizeof(float2) * (size_t)n);
     LogLayout l{reinterpret_cast<EdgeRow*>(scratch + rows), reinterpret_cast<EdgeHalf*>(scratch + third),
-                reinterpret_cast<float2*>(scratch + cen), scratch + logs, n <= kPackedLogNodes, 0};
-    if (logs < kScratchBytes)
-        l.slots = (long long)((kScratchBytes - logs) / ((l.packed ? 6 : sizeof(int4)) * (size_t)n));
+                reinterpret_cast<float2*>(scratch + cen), scratch + logs, n <= kPackedLogNodes ? 6 : 8, 0};
+    if (logs < kScratchBytes) l.slots = (long long)((kScratchBytes - logs) / (l.entry * (size_t)n));
     return l;
 }
+
+static_assert(kScratchBytes / (sizeof(EdgeRow) * 4) <= kHalfLogNodes, "log_layout: larger navmeshes have no slots");
 
 size_t smem_per_warp(int T, int C) { return (size_t)4 * kEntry * T * (C + 3); }
 
@@ -597,7 +599,7 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
         p.C = C;
         p.K = heuristic_k;
         p.log = lay.logs;
-        p.log_packed = lay.packed;
+        p.log_bytes = lay.entry;
         p.slots = blocks_log;
         p.work_ctr = reinterpret_cast<int*>(ds->scratch + kWorkOff);
         p.max_rounds = a.max_rounds;

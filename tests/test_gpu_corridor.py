@@ -111,7 +111,7 @@ def test_noalloc_log_form(lib, oracle_mod, T, Cap):
 
 @pytest.mark.parametrize("n", [0x7fc0, 0x7fc1])
 def test_noalloc_log_entry_sizes(lib, oracle_mod, n):
-    # the largest navmesh with 6-byte log entries and the smallest with 16: ids,
+    # the largest navmesh with 6-byte log entries and the smallest with 8: ids,
     # log places and depths (searches of a triangle nobody lists run to the
     # strip's other end) up to the ends of their fields
     import ctypes as C

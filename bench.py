@@ -220,7 +220,7 @@ def issue_roofline(rounds: int, search_ms: float, ipr, src, sm_mhz, sms: int):
     mhz = sm_mhz or 1965.0
     achieved = rounds * ipr / (search_ms / 1e3) / 1e9
     peak = 4 * sms * mhz / 1e3
-    return {"bound": "issue", "kernel": "k_search", "achieved": achieved, "peak": peak,
+    return {"bound": "issue", "kernel": "k_corridor_search", "achieved": achieved, "peak": peak,
             "unit": "G warp instructions/s", "frac": achieved / peak, "inst_per_round": ipr,
             "inst_source": src, "peak_basis": f"4 schedulers x {sms} SMs x {mhz:.0f} MHz (sampled SM clock)"}
 
@@ -593,7 +593,7 @@ def longest_query(g, starts, targets, torch):
 
 
 def mover_roofline(stats, A, peak, peak_kind):
-    """The mover phase (k_move_bin, k_cell_scan, k_scatter, k_collide_progress)
+    """The mover phase (k_move_bin, k_collide_progress)
     against HBM: per agent per frame 64 + 16 B plus 8 B per agent read from
     the 3x3 grid cells (the `neighbours` counter), over the mover's CUDA-event
     time of the frames in which agents moved."""
@@ -603,7 +603,7 @@ def mover_roofline(stats, A, peak, peak_kind):
     byt = sum(80.0 * A + 8.0 * s["neighbours"] for s in fr)
     ms = sum(s["ms_mover"] for s in fr)
     achieved = byt / (ms / 1e3) / 1e9
-    return {"bound": "hbm", "kernels": "k_move_bin + k_cell_scan + k_scatter + k_collide_progress",
+    return {"bound": "hbm", "kernels": "k_move_bin + k_collide_progress",
             "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
             "algorithmic_bytes_per_frame": byt / len(fr), "mover_ms_per_frame": ms / len(fr),
             "neighbours_per_agent": sum(s["neighbours"] for s in fr) / (len(fr) * A), "frames": len(fr)}
@@ -885,7 +885,7 @@ def bench_b200(args):
             "e2e_step_ms_over_many_frames": p99_long,
             "e2e_attribution": attribution(wall, parts),
             "e2e_sequential": e2e_seq,
-            "roofline": {"bound": "hbm", "kernel": "k_search", "achieved": achieved, "peak": peak,
+            "roofline": {"bound": "hbm", "kernel": "k_corridor_search", "achieved": achieved, "peak": peak,
                          "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "traffic_source": traffic_src,
                          "search_ms_per_step": statistics.mean(search_ms),
@@ -990,7 +990,7 @@ def timeline_summary(tl: np.ndarray, slots: int) -> dict:
 
 
 def profile_search(spec: str, budget_mb: int, timeline: bool):
-    """One batch search on a seeded maze, for profilers (ncu -k k_search):
+    """One batch search on a seeded maze, for profilers (ncu -k k_corridor_search):
     spec = "CELLS,T,C,VISITED_MODE,QUERIES".  Builds the CELLS x CELLS maze of
     the batched-uneven-queries configuration, draws QUERIES seeded free-space
     start/target pairs (numpy default_rng(7), starts then targets) and runs

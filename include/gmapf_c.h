@@ -95,7 +95,10 @@ typedef struct gmapf_options {
                                   tail), moves its bitmap into their shared memory (the bitmap, N/4 bytes for
                                   N triangles, has to fit in one block's shared memory; automatic
                                   placement only picks 4 where it does, a forced 4 that does not fit
-                                  fails the start with GMAPF_E_CAPACITY) */
+                                  fails the start with GMAPF_E_CAPACITY).  On maps of long thin corridors
+                                  1 and 4 also select the search kernel made for those (and claim
+                                  logs of 16 bytes per triangle and slot instead of 32-byte records);
+                                  results are the same with every value */
     int32_t path_smoothing;    /* 1: agents steer through the corridor's funnel corners (portal edges)
                                   instead of triangle centroids; 2: the same with every portal narrowed
                                   by the agent radius at both ends, so the corners keep that clearance

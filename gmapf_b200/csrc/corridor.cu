@@ -103,11 +103,11 @@ static_assert(kHalfLogNodes <= 1 << 20, "HalfLog: an edge has 22 bits, an entry 
 
 // In 6 bytes, for maps of at most kPackedLogNodes triangles: a word of the edge (17
 // bits) and parent + 1 (15; an ancestor is an earlier claim), a half word of
-// jump + 1.  2.7 times the searches of WideLog in a fixed scratch array (searches without allocation).
-// Where memory is not the limit the wide entry costs fewer instructions: 64x64-cell
-// maze, placement 1, packed in 8 bytes, 16,384 searches at T=4 14.5 against 14.9
-// ms, T=8 6.9 against 7.0, 37 searches 0.575 against 0.603; at T=32 the packed one
-// was 0-6% faster, within what its runs differ by.
+// jump + 1.  2.7 times the searches of WideLog in a fixed scratch array (searches
+// without allocation).  Where memory is not the limit the wide entry costs fewer
+// instructions: 64x64-cell maze, placement 1, against entries of 8 bytes, 16,384
+// searches at T=4 14.5 to 14.9 ms, T=8 6.9 to 7.0, 37 searches 0.575 to 0.603; at
+// T=32 the packed one was 0-6% faster, within what its runs differ by.
 struct PackedLog {
     unsigned* p;         // slots x n words, then slots x n half words
     unsigned short* pj;

@@ -488,7 +488,7 @@ int device_start(Context& c, std::string& err) {
 
     const HostMap& m = c.map;
     const int n = m.n;
-    if (c.scenes.empty()) c.scenes.push_back(single_scene(c));
+    if (!c.is_world) c.scenes.assign(1, single_scene(c));  // (agents may have come since a start that failed)
     const int nsc = (int)c.scenes.size();
     int max_scene_n = 1;
     for (const SceneInfo& si : c.scenes) max_scene_n = std::max(max_scene_n, si.n);
@@ -654,33 +654,21 @@ void device_free(Context& c) {
     destroy_graph(c);
     for (void* p : d.allocs)
         if (p) cudaFree(p);
-    d.allocs.clear();
-    d.rec = nullptr;  // freed above: a later start allocates anew
-    d.epoch = nullptr;
-    d.log = nullptr;
-    d.queues = nullptr;
-    d.queue_cap = 0;
-    d.gbm = nullptr;
-    d.rec_cap = d.log_cap = d.gbm_cap = 0;
-    d.slots = 0;
     for (auto& e : d.ev)
-        if (e) cudaEventDestroy(e), e = nullptr;
+        if (e) cudaEventDestroy(e);
     if (d.frame_done) cudaEventDestroy(d.frame_done);
-    d.frame_done = nullptr;
     if (d.stream) cudaStreamDestroy(d.stream);
     if (d.stream2) cudaStreamDestroy(d.stream2);
-    d.stream = d.stream2 = nullptr;
     if (d.loc_stream) cudaStreamSynchronize(d.loc_stream), cudaStreamDestroy(d.loc_stream);
     if (d.loc_pts) cudaFree(d.loc_pts);
     if (d.loc_node) cudaFree(d.loc_node);
     if (d.h_loc_pts) cudaFreeHost(d.h_loc_pts);
     if (d.h_loc_node) cudaFreeHost(d.h_loc_node);
-    d.loc_stream = nullptr;
-    d.loc_pts = nullptr;
-    d.loc_node = nullptr;
-    d.h_loc_pts = nullptr;
-    d.h_loc_node = nullptr;
-    d.loc_cap = 0;
+    // a later start (this one may have failed) allocates and sizes anew, and
+    // only what its own options ask for: nothing of this one may stay set
+    const int device = d.device;
+    d = Device{};
+    d.device = device;
     void* hp[] = {c.h_frame, c.h_dirty, c.h_step};
     for (void* p : hp)
         if (p) cudaFreeHost(p);

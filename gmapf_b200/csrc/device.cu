@@ -269,12 +269,35 @@ int pick_slots(Context& c, int& blocks, std::string& err) {
     long long best_slots = 0;
     const int want_vm = c.opt.visited_mode ? c.opt.visited_mode : c.tuned_vm;
     const int want_bt = c.opt.block_threads ? c.opt.block_threads : c.tuned_bt;
+    auto consider = [&](int vm, int bt, int form) {  // true: it has room for a block
+        const int per_sm = search_max_blocks_per_sm(c.T, c.C, bt, vm, d.bm_words, form);
+        if (per_sm <= 0) return false;
+        const int gpb = bt / 32;  // one request slot per warp
+        long long slots = std::min((long long)sms * per_sm * gpb,
+                                   budget / (long long)search_slot_bytes(n, vm, d.bm_words, form));
+        slots = (slots / gpb) * gpb;
+        if (slots < gpb) return false;
+        const long long weight = form != FORM_RECORDS ? (vm == 1 ? 64 : 40) : (vm == 1 ? 40 : vm >= 3 ? 30 : 20);
+        long long score = 10 * slots * weight + (vm == 4 ? 1 : 0);
+        if (form == FORM_LOG_GLOBAL) score = score * 9 / 10;
+        if (score > best_score) {
+            best_score = score;
+            best_bt = bt;
+            best_vm = vm;
+            best_form = form;
+            best_slots = slots;
+        }
+        return true;
+    };
     for (int vm = 1; vm <= 4; vm++) {
         if (want_vm != 0 && want_vm != vm) continue;
         // the first of equal scores wins; placement 4 prefers 256-thread blocks
         // (measured faster than 128 on the 160x160 maze: 27.1 against 28.0 ms
         // for a frame batch)
-        const int bts3[4] = {128, 64, 32, 256}, bts4[4] = {256, 128, 64, 32};
+        std::vector<int> bts = vm == 4 ? std::vector<int>{256, 128, 64, 32} : std::vector<int>{128, 64, 32, 256};
+        bts.erase(std::remove_if(bts.begin(), bts.end(),
+                                 [&](int bt) { return (want_bt != 0 && bt != want_bt) || bt % c.T != 0; }),
+                  bts.end());
         // corridor.cu's kernel, the longer the corridors the sooner: T = 32 on 8-,
         // 12- and 24-cell mazes (84, 147 and 329 levels; 4,096 queries) 0.047,
         // 0.080, 0.18 ms against search.cu's 0.059, 0.094, 0.24; T = 8 0.074,
@@ -282,30 +305,21 @@ int pick_slots(Context& c, int& blocks, std::string& err) {
         // 0.120, 0.39, 1.25.  Between rectangles (8 to 49 levels) it is slower
         // as soon as the fronts fill the lanes: T = 8, 1,313 triangles, 0.121
         // against 0.096.
-        const bool log = (vm == 1 || vm == 4) && d.corridor_levels >= (c.T >= 16 ? 64 : 256);
-        for (int bt : (vm == 4 ? bts4 : bts3)) {
-            if (want_bt != 0 && bt != want_bt) continue;
-            if (bt % c.T) continue;
-            for (int form = log ? FORM_LOG : FORM_RECORDS; form <= (log ? FORM_LOG_GLOBAL : FORM_RECORDS); form++) {
-                const int per_sm = search_max_blocks_per_sm(c.T, c.C, bt, vm, d.bm_words, form);
-                if (per_sm <= 0) continue;
-                const int gpb = bt / 32;  // one request slot per warp
-                long long slots = std::min((long long)sms * per_sm * gpb,
-                                           budget / (long long)search_slot_bytes(n, vm, d.bm_words, form));
-                slots = (slots / gpb) * gpb;
-                if (slots < gpb) continue;
-                const long long weight = log ? (vm == 1 ? 64 : 40) : (vm == 1 ? 40 : vm >= 3 ? 30 : 20);
-                long long score = 10 * slots * weight + (vm == 4 ? 1 : 0);
-                if (form == FORM_LOG_GLOBAL) score = score * 9 / 10;
-                if (score > best_score) {
-                    best_score = score;
-                    best_bt = bt;
-                    best_vm = vm;
-                    best_form = form;
-                    best_slots = slots;
-                }
-            }
-        }
+        bool log = (vm == 1 || vm == 4) && d.corridor_levels >= (c.T >= 16 ? 64 : 256);
+        // A placement that was asked for is refused on every map alike: where search.cu's
+        // kernel has no room for it (corridor.cu's may, with its queues in global memory).
+        if (log && c.opt.visited_mode == vm)
+            log = std::any_of(bts.begin(), bts.end(), [&](int bt) {
+                return search_max_blocks_per_sm(c.T, c.C, bt, vm, d.bm_words, FORM_RECORDS) > 0;
+            });
+        bool placed = false;
+        if (log)
+            for (int bt : bts)
+                for (int form : {FORM_LOG, FORM_LOG_GLOBAL}) placed |= consider(vm, bt, form);
+        // (corridor.cu's kernel has a larger fixed share: search.cu's serves the maps
+        // whose bitmap just fits)
+        if (!placed)
+            for (int bt : bts) consider(vm, bt, FORM_RECORDS);
     }
     if (best_score < 0) {
         err = "search kernel cannot be resident with T=" + std::to_string(c.T) + " C=" +

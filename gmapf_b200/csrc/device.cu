@@ -233,7 +233,7 @@ CompactScenes compact_scenes(const Context& c) {
     return CompactScenes{d.agent_scene, d.scene_abase, d.scene_P, d.scene_first};
 }
 
-int pick_slots(Context& c, int& blocks, std::string& err) {
+int pick_slots(Context& c, int& blocks, long long& budget, std::string& err) {
     Device& d = c.dev;
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d.device));
@@ -243,8 +243,8 @@ int pick_slots(Context& c, int& blocks, std::string& err) {
     // reuses or replaces it
     const int n = std::max(1, c.map.n);
     freeb += (size_t)d.rec_cap * (sizeof(Rec) * n + sizeof(unsigned)) + (size_t)d.log_cap * sizeof(int4) * n +
-             (size_t)d.gbm_cap * 4 * (size_t)d.bm_words;
-    long long budget = c.opt.search_mem_budget > 0 ? c.opt.search_mem_budget : (40ll << 30);
+             d.queue_cap + (size_t)d.gbm_cap * 4 * (size_t)d.bm_words;
+    budget = c.opt.search_mem_budget > 0 ? c.opt.search_mem_budget : (40ll << 30);
     budget = std::min<long long>(budget, (long long)(freeb * 0.6));
     d.bm_words = search_bitmap_words(n);
 
@@ -274,7 +274,7 @@ int pick_slots(Context& c, int& blocks, std::string& err) {
         if (per_sm <= 0) return false;
         const int gpb = bt / 32;  // one request slot per warp
         long long slots = std::min((long long)sms * per_sm * gpb,
-                                   budget / (long long)search_slot_bytes(n, vm, d.bm_words, form));
+                                   budget / (long long)search_slot_bytes(n, vm, d.bm_words, form, c.T, c.C));
         slots = (slots / gpb) * gpb;
         if (slots < gpb) return false;
         const long long weight = form != FORM_RECORDS ? (vm == 1 ? 64 : 40) : (vm == 1 ? 40 : vm >= 3 ? 30 : 20);
@@ -348,19 +348,35 @@ void release(Context& c, void* p) {
     cudaFree(p);
 }
 
-// Search state for the shape in c (T, C, visited placement, block size).
-// The record, log, queue and bitmap arrays are kept while the new shape's slots
-// fit them (the autotuner reshapes a hundred times; a ~12 GB free, allocation
-// and clear each time would take seconds).  Reuse needs no clearing: slot s
-// keeps its records together with its query epoch, so an old stamp never
-// equals a new epoch (modes 1 and 3 stamp 0, which no mode-2 epoch is), a
-// search reads only the log and queue entries it wrote, and the bitmaps are
-// cleared at the start of every query.
-int alloc_search_state(Context& c, std::string& err) {
+// the arrays of the search state that the sized search does not use (all: every one)
+void trim_search_state(Context& c, bool all = false) {
     Device& d = c.dev;
-    int blocks = 0;
-    int rc = pick_slots(c, blocks, err);
-    if (rc) return rc;
+    if (all || d.form != FORM_RECORDS) {
+        release(c, d.rec);
+        release(c, d.epoch);
+        d.rec = nullptr;
+        d.epoch = nullptr;
+        d.rec_cap = 0;
+    }
+    if (all || d.form == FORM_RECORDS) {
+        release(c, d.log);
+        d.log = nullptr;
+        d.log_cap = 0;
+    }
+    if (all || d.form != FORM_LOG_GLOBAL) {
+        release(c, d.queues);
+        d.queues = nullptr;
+        d.queue_cap = 0;
+    }
+    if (all || d.vm < 3) {
+        release(c, d.gbm);
+        d.gbm = nullptr;
+        d.gbm_cap = 0;
+    }
+}
+
+int alloc_search_arrays(Context& c, std::string& err) {
+    Device& d = c.dev;
     const size_t n = std::max(1, c.map.n);
     if (d.form == FORM_RECORDS && (!d.rec || d.slots > d.rec_cap)) {
         release(c, d.rec);
@@ -399,23 +415,38 @@ int alloc_search_state(Context& c, std::string& err) {
     return GMAPF_OK;
 }
 
-// after the shape is settled: the arrays of the other kernel's trials go
-void trim_search_state(Context& c) {
+// Search state for the shape in c (T, C, visited placement, block size).
+// The record, log, queue and bitmap arrays are kept while the new shape's slots
+// fit them and all of them together stay within the budget (the autotuner
+// reshapes a hundred times, from one kernel to the other; a ~12 GB free,
+// allocation and clear each time would take seconds).  Reuse needs no clearing: slot s
+// keeps its records together with its query epoch, so an old stamp never
+// equals a new epoch (modes 1 and 3 stamp 0, which no mode-2 epoch is), a
+// search reads only the log and queue entries it wrote, and the bitmaps are
+// cleared at the start of every query.
+int alloc_search_state(Context& c, std::string& err) {
     Device& d = c.dev;
-    if (d.form == FORM_RECORDS) {
-        release(c, d.log);
-        release(c, d.queues);
-        d.log = nullptr;
-        d.queues = nullptr;
-        d.log_cap = 0;
-        d.queue_cap = 0;
-    } else {
-        release(c, d.rec);
-        release(c, d.epoch);
-        d.rec = nullptr;
-        d.epoch = nullptr;
-        d.rec_cap = 0;
+    int blocks = 0;
+    long long budget = 0;
+    int rc = pick_slots(c, blocks, budget, err);
+    if (rc) return rc;
+    const size_t n = std::max(1, c.map.n);
+    auto held = [&]() {  // by the arrays once they are sized
+        const bool rec = d.form == FORM_RECORDS, global = d.form == FORM_LOG_GLOBAL;
+        const size_t queues = global ? d.slots * corridor_queue_bytes(c.C, c.T) : 0;
+        return (long long)(std::max(d.rec_cap, rec ? d.slots : 0) * sizeof(Rec) * n +
+                           std::max(d.log_cap, rec ? 0 : d.slots) * sizeof(int4) * n + std::max(d.queue_cap, queues) +
+                           std::max(d.gbm_cap, d.vm >= 3 ? d.slots : 0) * 4 * (size_t)d.bm_words);
+    };
+    if (held() > budget) trim_search_state(c);
+    if (held() > budget) trim_search_state(c, true);
+    rc = alloc_search_arrays(c, err);
+    if (rc == GMAPF_E_CAPACITY) {  // (what is kept may be in the way)
+        err.clear();
+        trim_search_state(c, true);
+        rc = alloc_search_arrays(c, err);
     }
+    return rc;
 }
 
 int search_blocks(Context& c) { return c.dev.slots / (c.block_threads / 32); }
@@ -1062,7 +1093,9 @@ int device_apply_tuned_shape(Context& c, int T, int C, int vm, int bt, std::stri
     c.C = C;
     c.tuned_vm = vm;
     c.tuned_bt = bt;
-    return device_reconfigure_search(c, err);
+    const int rc = device_reconfigure_search(c, err);
+    if (rc == GMAPF_OK) trim_search_state(c);
+    return rc;
 }
 
 // Per-map autotuner (batched form): threads per agent T, queue capacity C,

@@ -228,8 +228,8 @@ cudaError_t launch_search(cudaStream_t s, const SearchParams& p, int blocks, int
 // which kernel a search runs on: search.cu's, with a record per claimed node,
 // or corridor.cu's, with a claim log, its queues in shared or in global memory
 enum SearchForm { FORM_RECORDS = 0, FORM_LOG, FORM_LOG_GLOBAL };
-// device memory of one request slot: records or claim log, and visited state
-size_t search_slot_bytes(int n_nodes, int vm, int bm_words, int form);
+// device memory of one request slot: records or claim log, queues, visited state
+size_t search_slot_bytes(int n_nodes, int vm, int bm_words, int form, int T, int C);
 size_t search_smem_bytes(int C, int block_threads, int bm_words, int T, int vm);
 int search_bitmap_words(int n_nodes);
 int search_max_blocks_per_sm(int T, int C, int block_threads, int vm, int bm_words, int form);

@@ -840,8 +840,9 @@ int search_bitmap_words(int n_nodes) {
     return (w + 3) & ~3;  // whole uint4 for the clear
 }
 
-size_t search_slot_bytes(int n_nodes, int vm, int bm_words, int form) {
-    return (form == FORM_RECORDS ? sizeof(Rec) : sizeof(int4)) * (size_t)n_nodes + (vm >= 3 ? 4 * (size_t)bm_words : 0);
+size_t search_slot_bytes(int n_nodes, int vm, int bm_words, int form, int T, int C) {
+    return (form == FORM_RECORDS ? sizeof(Rec) : sizeof(int4)) * (size_t)n_nodes +
+           (form == FORM_LOG_GLOBAL ? corridor_queue_bytes(C, T) : 0) + (vm >= 3 ? 4 * (size_t)bm_words : 0);
 }
 
 int search_max_blocks_per_sm(int T, int C, int bt, int vm, int bm_words, int form) {

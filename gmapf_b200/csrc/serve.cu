@@ -441,7 +441,7 @@ int serve_start(Context& c, int max_in_flight, std::string& err) {
         err = "serving: the search kernel cannot be resident with this shape";
         return GMAPF_E_CAPACITY;
     }
-    const double per_slot = (double)search_slot_bytes(n, d.vm, d.bm_words, d.form);
+    const double per_slot = (double)search_slot_bytes(n, d.vm, d.bm_words, d.form, c.T, c.C);
     // the drain launch is persistent while queries keep coming: leave one
     // block per SM for the frames' own kernels
     const int drain_per_sm = per_sm > 1 ? per_sm - 1 : 1;

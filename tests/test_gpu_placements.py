@@ -54,3 +54,20 @@ def test_queues_that_leave_no_room(vm):
     with pytest.raises(G.GMAPFError, match="E_CAPACITY"):
         start(long_strip(200_000), 32, 512, visited_mode=vm)
     assert start(long_strip(200_000), 32, 512).search_shape()["slots"] > 0
+
+
+@pytest.mark.parametrize("options", [{}, dict(autotune=True), dict(visited_mode=4)])
+def test_search_memory_within_its_budget(options):
+    # T=32, C=256: 98,304 bytes of queues to 32,000 of claim log in a slot
+    import torch
+    nodes, budget = long_strip(2000), 64 << 20
+    start(nodes, 32, 256, **options).close()  # (what the process keeps is there)
+
+    def held(budget):
+        before = torch.cuda.mem_get_info()[0]
+        g = start(nodes, 32, 256, search_mem_budget=budget, **options)
+        used = before - torch.cuda.mem_get_info()[0]
+        g.close()
+        return used
+
+    assert held(budget) - held(1 << 20) <= budget + (8 << 20)  # (2 MiB granules)

@@ -54,7 +54,7 @@ int search_promote_rounds(const Context& c) { return c.opt.promote_rounds > 0 ? 
 namespace {
 
 // device counters: [8] holds the frame's dt as a float
-enum Counter { CT_REQ = 0, CT_MOVE = 1, CT_WORK = 2, CT_ERR = 3, CT_ERR_TARGETS = 4, CT_PARITY = 9 /* and 10 */, CT_COUNT = 16 };
+enum Counter { CT_REQ = 0, CT_MOVE = 1, CT_WORK = 2, CT_ERR = 3, CT_ERR_TARGETS = 4, CT_PARITY = 9 /* and 10 */, CT_COUNT = kCounters };
 
 template <class T>
 int dalloc(Context& c, T** p, size_t count, std::string& err) {
@@ -556,23 +556,19 @@ int device_start(Context& c, std::string& err) {
 
     // agents
     const int A = c.A;
-    // what a frame brings back to the host, in one buffer and one copy:
-    // positions, states, counters, statistics
-    const size_t at_state = (sizeof(float2) * A + 15) & ~(size_t)15;
-    const size_t at_counters = (at_state + sizeof(int) * A + 15) & ~(size_t)15;
-    const size_t at_stats = at_counters + sizeof(int) * CT_COUNT;
-    d.frame_bytes = at_stats + sizeof(unsigned long long) * ST_COUNT;
+    const FrameLayout at(A);
+    d.frame_bytes = at.bytes;
     DALLOC(d.frame, d.frame_bytes);
     d.pos = reinterpret_cast<float2*>(d.frame);
-    d.state = reinterpret_cast<int*>(d.frame + at_state);
-    d.counters = reinterpret_cast<int*>(d.frame + at_counters);
-    d.stats = reinterpret_cast<unsigned long long*>(d.frame + at_stats);
+    d.state = reinterpret_cast<int*>(d.frame + at.state);
+    d.counters = reinterpret_cast<int*>(d.frame + at.counters);
+    d.stats = reinterpret_cast<unsigned long long*>(d.frame + at.stats);
     CK(cudaMallocHost((void**)&c.h_frame, d.frame_bytes));
     std::memset(c.h_frame, 0, d.frame_bytes);
     c.h_pos_stage = reinterpret_cast<float2*>(c.h_frame);
-    c.h_state_stage = reinterpret_cast<int*>(c.h_frame + at_state);
-    c.h_small = reinterpret_cast<int*>(c.h_frame + at_counters);
-    c.h_stats = reinterpret_cast<unsigned long long*>(c.h_frame + at_stats);
+    c.h_state_stage = reinterpret_cast<int*>(c.h_frame + at.state);
+    c.h_small = reinterpret_cast<int*>(c.h_frame + at.counters);
+    c.h_stats = reinterpret_cast<unsigned long long*>(c.h_frame + at.stats);
     DALLOC(d.pos_mid, A);
     DALLOC(d.targ_pos, A);
     DALLOC(d.step_pos, A);
@@ -1002,8 +998,8 @@ int device_search_batch(Context& c, const int* d_starts, const int* d_targets, i
         }
     }
     CK(cudaEventRecord(d.ev[7], s));
-    CK(cudaMemcpyAsync(c.h_small, d.counters, sizeof(int) * CT_COUNT + sizeof(unsigned long long) * ST_COUNT,
-                       cudaMemcpyDeviceToHost, s));  // (the statistics follow the counters)
+    const FrameLayout at(c.A);
+    CK(cudaMemcpyAsync(c.h_small, d.counters, at.bytes - at.counters, cudaMemcpyDeviceToHost, s));  // (and the statistics)
     CK(cudaStreamSynchronize(s));
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, d.ev[6], d.ev[7]));

@@ -298,6 +298,24 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+// What a frame brings back to the host, in one buffer and one copy: positions,
+// states, counters, statistics (byte offsets).  Counters and statistics have
+// 256-byte lines of their own: searches take their next request from a counter
+// while others add to the statistics, and atomics on one line wait for one
+// another (16,384 searches in 62 triangles, T=32: 0.107 ms with both in one
+// line, 0.078 apart).
+constexpr int kCounters = 16;
+struct FrameLayout {
+    size_t state, counters, stats, bytes;
+    explicit FrameLayout(int agents) {
+        auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+        state = up(sizeof(float2) * (size_t)agents);
+        counters = up(state + sizeof(int) * (size_t)agents);
+        stats = up(counters + sizeof(int) * kCounters);
+        bytes = stats + sizeof(unsigned long long) * ST_COUNT;
+    }
+};
+
 struct Device {
     int device = 0;
     cudaStream_t stream = nullptr, stream2 = nullptr;

@@ -298,14 +298,7 @@ int pick_slots(Context& c, int& blocks, long long& budget, std::string& err) {
         bts.erase(std::remove_if(bts.begin(), bts.end(),
                                  [&](int bt) { return (want_bt != 0 && bt != want_bt) || bt % c.T != 0; }),
                   bts.end());
-        // corridor.cu's kernel, the longer the corridors the sooner: T = 32 on 8-,
-        // 12- and 24-cell mazes (84, 147 and 329 levels; 4,096 queries) 0.047,
-        // 0.080, 0.18 ms against search.cu's 0.059, 0.094, 0.24; T = 8 0.074,
-        // 0.20, 0.63 against 0.074, 0.20, 0.69; T = 4 0.135, 0.44, 1.21 against
-        // 0.120, 0.39, 1.25.  Between rectangles (8 to 49 levels) it is slower
-        // as soon as the fronts fill the lanes: T = 8, 1,313 triangles, 0.121
-        // against 0.096.
-        bool log = (vm == 1 || vm == 4) && d.corridor_levels >= (c.T >= 16 ? 64 : 256);
+        bool log = (vm == 1 || vm == 4) && corridor_kernel_serves(d.corridors, c.T);
         // A placement that was asked for is refused on every map alike: where search.cu's
         // kernel has no room for it (corridor.cu's may, with its queues in global memory).
         if (log && c.opt.visited_mode == vm)
@@ -667,13 +660,15 @@ int device_start(Context& c, std::string& err) {
 
     // long corridors: the edge rows (144 bytes per triangle; a directed edge is an
     // int) where they take little of what is left, else search.cu serves all maps
-    d.corridor_levels = 0;
+    d.corridors = Corridors{};
     if (n > 0 && n <= (1 << 24)) {
         size_t freeb = 0, totalb = 0;
         CK(cudaMemGetInfo(&freeb, &totalb));
-        if (144 * (double)n <= 0.05 * (double)freeb) d.corridor_levels = corridor_levels(m, c.scenes);
+        if (144 * (double)n <= 0.05 * (double)freeb) d.corridors = measure_corridors(m, c.scenes);
     }
-    if (d.corridor_levels >= 64) {
+    bool thin = false;
+    for (int T : {2, 4, 8, 16, 32}) thin = thin || corridor_kernel_serves(d.corridors, T);
+    if (thin) {
         DALLOC(d.erow, 4 * (size_t)n);
         DALLOC(d.third, n);
         launch_edge_rows(d.stream, d.rows, n, d.erow, d.third);

@@ -167,22 +167,24 @@ static void bfs_hops(const HostMap& m, int src, std::vector<unsigned short>& d) 
     }
 }
 
-int corridor_levels(const HostMap& m, const std::vector<SceneInfo>& scenes) {
-    // levels and triangles of a breadth-first wave from each scene's first
-    // triangle or from the farthest one from it, whichever is longer
-    long long levels = 0, nodes = 0, waves = 0;
+Corridors measure_corridors(const HostMap& m, const std::vector<SceneInfo>& scenes) {
+    // a breadth-first wave from each scene's first triangle or from the farthest
+    // one from it, whichever has more levels
+    long long levels = 0, nodes = 0, loops = 0, waves = 0;
     std::vector<int> d(m.n, -1), q;
     for (const SceneInfo& si : scenes) {
         if (si.n == 0) continue;
         int src = si.node_base;
-        long long lv = 0, cnt = 0;
+        long long lv = 0, cnt = 0, lp = 0;
         for (int pass = 0; pass < 2; pass++) {
             for (int v : q) d[v] = -1;
             q.assign(1, src);
             d[src] = 0;
+            long long sides = 0;
             for (size_t h = 0; h < q.size(); h++) {
                 const SearchRow& r = m.rows[q[h]];
                 const int nb[3] = {r.n0, r.n1, r.n2};
+                sides += r.deg;
                 for (int k = 0; k < r.deg; k++)
                     if (d[nb[k]] < 0) {
                         d[nb[k]] = d[q[h]] + 1;
@@ -193,15 +195,44 @@ int corridor_levels(const HostMap& m, const std::vector<SceneInfo>& scenes) {
             if (d[src] + 1 > lv) {
                 lv = d[src] + 1;
                 cnt = (long long)q.size();
+                lp = std::max(0ll, sides / 2 - cnt);
             }
             // the second wave has at most twice the levels: often the first one tells
-            if ((lv >= 256 && cnt <= 16 * lv) || cnt > 32 * lv) break;
+            if ((lv >= 1000 && cnt <= 16 * lv && 20 * lp <= 9 * lv) || cnt > 32 * lv) break;
         }
         levels += lv;
         nodes += cnt;
+        loops += lp;
         waves++;
     }
-    return waves > 0 && nodes <= 16 * levels ? (int)(levels / waves) : 0;
+    Corridors c;
+    if (waves > 0 && nodes <= 16 * levels) {
+        c.levels = (int)(levels / waves);
+        c.loops = (float)((double)loops / (double)levels);
+    }
+    return c;
+}
+
+// Corridors of thin grids (w squares wide, 6,400 to 7,700 triangles, 4,096 queries),
+// mazes and braided mazes; search.cu's time over corridor.cu's:
+//   w (loops per level)   T=2     4     8    16    32
+//   1 (0)                1.08  1.29  1.30  1.59  1.38
+//   2 (0.5)              0.83  0.86  1.05  1.33  1.16
+//   3 (1.0)              0.72  0.74  0.75  1.30  1.05
+//   4 (1.55)             0.65  0.66  0.65  0.86  0.97 (512 queries 1.18)
+//   5 (2.0)              0.62  0.62  0.58  0.66  0.92
+//   8 (3.5)              0.61  0.57  0.55  0.62  0.55
+// A loop brings two of a round's candidates to one triangle: corridor.cu tells such
+// candidates apart one by one, search.cu all of them with one MATCH.ANY.  Long
+// mazes (64 x 64: 0.2 to 0.4 loops) 1.34 1.32 1.39 1.53 1.46; 20 to 28 cells a side (312 to
+// 492 levels) 0.90-0.95 0.91-1.04 1.00-1.13 1.33-1.43 1.17-1.23; 8 to 16 cells (84 to 225)
+// at T=16 and 32 1.03-1.15.  Braided mazes of 485 to 836 levels 0.77-1.05 0.83-1.22
+// 0.90-1.35 1.04-1.46 1.03-1.28: fewer threads per agent need longer corridors.
+// Between rectangles (8 to 49 levels, 2 to 4 loops) corridor.cu is the slower one.
+bool corridor_kernel_serves(const Corridors& c, int T) {
+    const int levels = T >= 16 ? 64 : T == 8 ? 256 : 1000;
+    const float loops = T == 32 ? 1.6f : T == 16 ? 1.1f : T == 8 ? 0.55f : 0.45f;
+    return c.levels >= levels && c.loops <= loops;
 }
 
 void landmark_distances(const HostMap& m, int count, std::vector<unsigned short>& out) {

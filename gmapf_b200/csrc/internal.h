@@ -282,10 +282,17 @@ void build_host_map(const gmapf_node* nodes, int n, HostMap& out);
 // global triangle ids; fills each scene's triangle range, bounds and
 // point-location grid (offsets into the concatenated grid arrays).
 void concat_host_maps(const std::vector<const HostMap*>& maps, HostMap& out, std::vector<SceneInfo>& scenes);
-// How long a map's corridors are: the levels of a breadth-first wave from a far
-// triangle (the mean over the scenes), 0 when the waves hold more than 16
-// triangles per level on average (open ground).
-int corridor_levels(const HostMap& m, const std::vector<SceneInfo>& scenes);
+// How long and how thin a map's corridors are: the levels of a breadth-first wave
+// from a far triangle (the mean over the scenes), 0 when the waves hold more than
+// 16 triangles per level on average (open ground), and how many loops the
+// neighbour graph closes per level.
+struct Corridors {
+    int levels = 0;
+    float loops = 0;
+};
+Corridors measure_corridors(const HostMap& m, const std::vector<SceneInfo>& scenes);
+// whether corridor.cu's kernel is the faster one there
+bool corridor_kernel_serves(const Corridors& c, int T);
 // Hop distances from `count` landmark triangles chosen by farthest-point
 // sampling over the neighbour graph (unreachable: 65535), count * n values.
 void landmark_distances(const HostMap& m, int count, std::vector<unsigned short>& out);
@@ -321,7 +328,7 @@ struct Device {
     cudaStream_t stream = nullptr, stream2 = nullptr;
     // map
     SearchRow* rows = nullptr;
-    int corridor_levels = 0;  // corridor_levels() of the map: long corridors are searched by corridor.cu's kernel
+    Corridors corridors;      // of the map: long thin ones are searched by corridor.cu's kernel
     EdgeRow* erow = nullptr;  // corridor maps: 4 per triangle
     EdgeHalf* third = nullptr;  // corridor maps: per triangle
     float2* cen = nullptr;

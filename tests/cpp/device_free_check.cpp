@@ -27,7 +27,8 @@ int main() {
     d.agent_scene = d.scene_abase = d.scene_P = d.scene_first = reinterpret_cast<int*>(buf);
     d.erow = reinterpret_cast<EdgeRow*>(buf);
     d.third = reinterpret_cast<EdgeHalf*>(buf);
-    d.corridor_levels = 300;
+    d.corridors.levels = 300;
+    d.corridors.loops = 0.5f;
     d.form = FORM_LOG_GLOBAL;
     d.full_pad = true;
     d.slots = d.rec_cap = d.log_cap = d.gbm_cap = 64;
@@ -57,7 +58,8 @@ int main() {
     GONE(scene_first);
     GONE(erow);
     GONE(third);
-    GONE(corridor_levels);
+    GONE(corridors.levels);
+    GONE(corridors.loops);
     GONE(form);
     GONE(full_pad);
     GONE(slots);

@@ -167,6 +167,23 @@ static void bfs_hops(const HostMap& m, int src, std::vector<unsigned short>& d) 
     }
 }
 
+// The neighbour graph's triangles reached from src, breadth first: order q, levels
+// d (-1 where none was, before and after).
+static void flood(const HostMap& m, int src, std::vector<int>& d, std::vector<int>& q) {
+    for (int v : q) d[v] = -1;
+    q.assign(1, src);
+    d[src] = 0;
+    for (size_t h = 0; h < q.size(); h++) {
+        const SearchRow& r = m.rows[q[h]];
+        const int nb[3] = {r.n0, r.n1, r.n2};
+        for (int k = 0; k < r.deg; k++)
+            if (d[nb[k]] < 0) {
+                d[nb[k]] = d[q[h]] + 1;
+                q.push_back(nb[k]);
+            }
+    }
+}
+
 Corridors measure_corridors(const HostMap& m, const std::vector<SceneInfo>& scenes) {
     // a breadth-first wave from each scene's first triangle or from the farthest
     // one from it, whichever has more levels
@@ -174,31 +191,41 @@ Corridors measure_corridors(const HostMap& m, const std::vector<SceneInfo>& scen
     std::vector<int> d(m.n, -1), q;
     for (const SceneInfo& si : scenes) {
         if (si.n == 0) continue;
-        int src = si.node_base;
+        flood(m, si.node_base, d, q);
+        if (2 * q.size() < (size_t)si.n) {
+            // a part of the scene cut off from the rest: the largest part decides, the
+            // one that most searches run in
+            std::vector<char> reached(si.n, 0);
+            int src = si.node_base, left = si.n;
+            size_t largest = 0;
+            for (int v = si.node_base; v < si.node_base + si.n && largest < (size_t)left; v++) {
+                if (reached[v - si.node_base]) continue;
+                flood(m, v, d, q);
+                for (int u : q) {
+                    char& r = reached[u - si.node_base];
+                    left -= !r;
+                    r = 1;
+                }
+                if (q.size() > largest) {
+                    largest = q.size();
+                    src = v;
+                }
+            }
+            flood(m, src, d, q);
+        }
         long long lv = 0, cnt = 0, lp = 0;
         for (int pass = 0; pass < 2; pass++) {
-            for (int v : q) d[v] = -1;
-            q.assign(1, src);
-            d[src] = 0;
-            long long sides = 0;
-            for (size_t h = 0; h < q.size(); h++) {
-                const SearchRow& r = m.rows[q[h]];
-                const int nb[3] = {r.n0, r.n1, r.n2};
-                sides += r.deg;
-                for (int k = 0; k < r.deg; k++)
-                    if (d[nb[k]] < 0) {
-                        d[nb[k]] = d[q[h]] + 1;
-                        q.push_back(nb[k]);
-                    }
-            }
-            src = q.back();  // a farthest one
-            if (d[src] + 1 > lv) {
-                lv = d[src] + 1;
+            const int far = q.back();  // a farthest one
+            if (d[far] + 1 > lv) {
+                long long sides = 0;
+                for (int v : q) sides += m.rows[v].deg;
+                lv = d[far] + 1;
                 cnt = (long long)q.size();
                 lp = std::max(0ll, sides / 2 - cnt);
             }
             // the second wave has at most twice the levels: often the first one tells
-            if ((lv >= 1000 && cnt <= 16 * lv && 20 * lp <= 9 * lv) || cnt > 32 * lv) break;
+            if (pass == 1 || (lv >= 1000 && cnt <= 16 * lv && 20 * lp <= 9 * lv) || cnt > 32 * lv) break;
+            flood(m, far, d, q);
         }
         levels += lv;
         nodes += cnt;

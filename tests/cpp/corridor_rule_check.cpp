@@ -77,7 +77,27 @@ static void expect(const char* what, const std::vector<gmapf_node>& nodes, const
     }
 }
 
+// two maps in one, cut off from one another
+static std::vector<gmapf_node> both(std::vector<gmapf_node> a, const std::vector<gmapf_node>& b) {
+    const int base = (int)a.size();
+    for (gmapf_node n : b) {
+        for (int& k : n.NeibsIdx)
+            if (k >= 0) k += base;
+        a.push_back(n);
+    }
+    return a;
+}
+
 int main() {
+    const auto open = squares(std::vector<std::vector<char>>(60, std::vector<char>(60, 1)));
+    const auto patch = squares(std::vector<std::vector<char>>(3, std::vector<char>(3, 1)));
+    const auto lane = squares(winding(1, 50, 1)), lanes = squares(winding(1, 160, 24));
+    expect("open ground", open, {});
+    expect("a lane, then open ground", both(lane, open), {});
+    expect("a patch and a lane, then open ground", both(both(patch, lane), open), {});
+    expect("a patch, then long lanes", both(patch, lanes), {2, 4, 8, 16, 32});
+    expect("open ground, then long lanes", both(open, lanes), {2, 4, 8, 16, 32});
+    expect("long lanes, then a patch", both(lanes, patch), {2, 4, 8, 16, 32});
     expect("1 wide", squares(winding(1, 160, 24)), {2, 4, 8, 16, 32});
     expect("2 wide", squares(winding(2, 160, 12)), {8, 16, 32});
     expect("3 wide", squares(winding(3, 160, 8)), {16, 32});

@@ -461,7 +461,7 @@ int enqueue_frame(Context& c, bool timing, std::string& err) {
     if (timing) CK(cudaEventRecordWithFlags(d.ev[0], s, cudaEventRecordExternal));
     launch_compact(s, c.A, d.state, d.cur, d.targ, c.cfg.PathFinderParallelAgents, compact_scenes(c), d.req,
                    d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_PARITY,
-                   d.counters + CT_WORK, d.order_hist, d.stats, frame_words(c));
+                   d.counters + CT_WORK, d.order_hist, d.stats, frame_words(c), c.serve != nullptr);
     if (timing) CK(cudaEventRecordWithFlags(d.ev[1], s, cudaEventRecordExternal));
     CK(cudaEventRecord(d.ev[5], s));
     CK(cudaStreamWaitEvent(s2, d.ev[5], 0));
@@ -717,6 +717,8 @@ void device_free(Context& c) {
     c.h_step = nullptr;
 }
 
+void device_drop_graph(Context& c) { destroy_graph(c); }
+
 int device_async_step(Context& c, float dt, std::string& err) {
     Device& d = c.dev;
     cudaStream_t s = d.stream;
@@ -754,7 +756,7 @@ int device_async_step(Context& c, float dt, std::string& err) {
         if (timing) CK(cudaEventRecord(d.ev[0], s));
         launch_compact(s, c.A, d.state, d.cur, d.targ, c.cfg.PathFinderParallelAgents, compact_scenes(c), d.req,
                        d.counters + CT_REQ, d.in_move, d.counters + CT_MOVE, d.counters + CT_PARITY,
-                       d.counters + CT_WORK, d.order_hist, d.stats, frame_words(c));
+                       d.counters + CT_WORK, d.order_hist, d.stats, frame_words(c), c.serve != nullptr);
         c.launches += 1;
         CK(cudaMemcpyAsync(c.h_small, d.counters, sizeof(int) * CT_COUNT, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));

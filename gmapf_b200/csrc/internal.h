@@ -189,7 +189,8 @@ struct FrameWords {
 };
 void launch_compact(cudaStream_t s, int A, int* state, const int* cur, const int* targ, int P,
                     const CompactScenes& scn, int4* req, int* req_count, unsigned char* in_move, int* mv_count,
-                    int* parity, int* work_ctr, int* hist, unsigned long long* stats, const FrameWords& words);
+                    int* parity, int* work_ctr, int* hist, unsigned long long* stats, const FrameWords& words,
+                    bool beside_searches);
 void launch_apply_targets(cudaStream_t s, const int4* recs, int n, int* state, int* targ_node,
                           float2* targ_pos);
 // device-resident retargets of agents id_base + ids[k], ids[k] in [0, id_count)
@@ -486,6 +487,8 @@ int search_promote_rounds(const Context& c);
 std::string device_error_text(int e);
 int device_start(Context& c, std::string& err);
 void device_free(Context& c);
+// the frame's graph is recorded anew by the next frame (its kernels' shapes change)
+void device_drop_graph(Context& c);
 int device_async_step(Context& c, float dt, std::string& err);
 int device_wait_step(Context& c, std::string& err);
 bool device_step_ready(Context& c);

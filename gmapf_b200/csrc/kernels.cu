@@ -28,10 +28,12 @@ namespace cg = cooperative_groups;
 
 constexpr int kOrderBuckets = 1024;  // of the longest-first order
 constexpr int kCompactThreads = 1024;
+constexpr int kBesideThreads = 256;  // beside served searches
 constexpr int kCompactRun = 4;       // consecutive agents per thread and step
 constexpr int kCompactCluster = 8;   // thread blocks (one cluster) for more agents than one block's step
 
-// inclusive block scan (1,024 threads) of v; *total gets the sum.  warp_tot: 32 words
+// inclusive block scan (TH threads) of v; *total gets the sum.  warp_tot: 32 words
+template <int TH>
 __device__ __forceinline__ int block_scan(int v, int* warp_tot, int* total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int o = 1; o < 32; o <<= 1) {
@@ -41,8 +43,8 @@ __device__ __forceinline__ int block_scan(int v, int* warp_tot, int* total) {
     __syncthreads();  // the previous scan's totals are read
     if (lane == 31) warp_tot[warp] = v;
     __syncthreads();
-    int w = warp_tot[lane];
-    for (int o = 1; o < 32; o <<= 1) {  // (every warp scans the 32 totals: no second barrier)
+    int w = TH == 1024 || lane < TH / 32 ? warp_tot[lane] : 0;
+    for (int o = 1; o < 32; o <<= 1) {  // (every warp scans the totals: no second barrier)
         const int t = __shfl_up_sync(0xffffffffu, w, o);
         if (lane >= o) w += t;
     }
@@ -53,10 +55,10 @@ __device__ __forceinline__ int block_scan(int v, int* warp_tot, int* total) {
 
 // block_scan over the cluster's blocks (CL of them) in rank order; cluster_tot:
 // CL words of shared memory, read by the other blocks
-template <int CL>
+template <int CL, int TH>
 __device__ __forceinline__ int cluster_scan(int v, int* warp_tot, int* cluster_tot, int* total) {
     int tot;
-    const int incl = block_scan(v, warp_tot, &tot);
+    const int incl = block_scan<TH>(v, warp_tot, &tot);
     if constexpr (CL == 1) {
         *total = tot;
         return incl;
@@ -87,10 +89,17 @@ __device__ __forceinline__ int cluster_scan(int v, int* warp_tot, int* cluster_t
 // one agent per thread and three barriers per scan took 29 and 63 us; the same
 // block with 16 agents per thread 34 and 23 us.)
 //
+// While a context serves, the blocks have 256 threads (1,024 agents a step in one
+// block, 8,192 in the cluster): a frame starts while searches fill the SMs, and
+// what serving leaves of an SM, one search block's share (24,576 registers beside
+// blocks of 256, 14,336 beside blocks of 128), has room for 256 threads of 49
+// registers, not for 1,024.  The frame after a burst of 8,192 retargets on the 64x64
+// maze at T=8 took 4.4 ms with blocks of 1,024 threads, 0.14 now.
+//
 // Per-scene request limits (a scene batch): scene s takes its Search agents in
 // ascending id up to P[s] (each scene is its own PathFinder, PathFinder.h:76-117).
 // first[s] records how many Search agents precede the scene's first agent.
-template <int CL>
+template <int CL, int TH>
 __device__ __forceinline__ void compact(int A, int* state, const int* cur, const int* targ, int P, const CompactScenes& scn,
                                         int4* req, int* req_count, unsigned char* in_move, int* mv_count, int* parity,
                                         int* work_ctr, int* hist, unsigned long long* stats, const FrameWords& words) {
@@ -99,12 +108,12 @@ __device__ __forceinline__ void compact(int A, int* state, const int* cur, const
     const int tid = threadIdx.x;
     const int rank = CL > 1 ? (int)blockIdx.x : 0;
     const bool scenes = scn.agent_scene != nullptr;
-    static_assert(kOrderBuckets == kCompactThreads, "one bucket per thread");
-    if (hist && rank == 0) hist[tid] = 0;  // the order's buckets
+    if (hist && rank == 0)  // the order's buckets
+        for (int k = tid; k < kOrderBuckets; k += TH) hist[k] = 0;
     const float dt = tid == 0 && rank == 0 ? *reinterpret_cast<const volatile float*>(words.dt_host) : 0.f;
     int base_s = 0, base_m = 0, base_o = 0;  // before this step (the same on every thread)
-    for (int b = 0; b < A; b += CL * kCompactThreads * kCompactRun) {
-        const int i0 = b + (rank * kCompactThreads + tid) * kCompactRun;
+    for (int b = 0; b < A; b += CL * TH * kCompactRun) {
+        const int i0 = b + (rank * TH + tid) * kCompactRun;
         const int cnt = max(0, min(kCompactRun, A - i0));
         int st[kCompactRun], cu[kCompactRun], ta[kCompactRun];
         if (cnt == kCompactRun) {  // (runs of 4 start on 16-byte boundaries)
@@ -143,7 +152,7 @@ __device__ __forceinline__ void compact(int A, int* state, const int* cur, const
         else
             for (int j = 0; j < cnt; j++) in_move[i0 + j] = (flags >> (8 * j)) & 1u;
         int tot;
-        const int incl = cluster_scan<CL>(ns | nm << 16, warp_tot, cluster_tot, &tot);
+        const int incl = cluster_scan<CL, TH>(ns | nm << 16, warp_tot, cluster_tot, &tot);
         int pos = base_s + (incl & 0xffff) - ns;  // Search agents before this run
         if (!scenes) {
 #pragma unroll
@@ -172,7 +181,7 @@ __device__ __forceinline__ void compact(int A, int* state, const int* cur, const
                 ok += want[j];
             }
             int tot_o;
-            int opos = base_o + cluster_scan<CL>(ok, warp_tot, cluster_tot, &tot_o) - ok;
+            int opos = base_o + cluster_scan<CL, TH>(ok, warp_tot, cluster_tot, &tot_o) - ok;
 #pragma unroll
             for (int j = 0; j < kCompactRun; j++)
                 if (want[j]) req[opos++] = make_int4(i0 + j, cu[j], ta[j], i0 + j);
@@ -201,12 +210,14 @@ __device__ __forceinline__ void compact(int A, int* state, const int* cur, const
 #define COMPACT_ARGS                                                                                          \
     int A, int *state, const int *cur, const int *targ, int P, CompactScenes scn, int4 *req, int *req_count, \
         unsigned char *in_move, int *mv_count, int *parity, int *work_ctr, int *hist, unsigned long long *stats, FrameWords words
-__global__ void __launch_bounds__(kCompactThreads) k_compact(COMPACT_ARGS) {
-    compact<1>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, parity, work_ctr, hist, stats, words);
+template <int TH>
+__global__ void __launch_bounds__(TH) k_compact(COMPACT_ARGS) {
+    compact<1, TH>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, parity, work_ctr, hist, stats, words);
 }
-__global__ void __cluster_dims__(kCompactCluster, 1, 1) __launch_bounds__(kCompactThreads)
+template <int TH>
+__global__ void __cluster_dims__(kCompactCluster, 1, 1) __launch_bounds__(TH, TH == kBesideThreads ? 5 : 1)
     k_compact_cluster(COMPACT_ARGS) {
-    compact<kCompactCluster>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, parity, work_ctr, hist, stats, words);
+    compact<kCompactCluster, TH>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count, parity, work_ctr, hist, stats, words);
 }
 #undef COMPACT_ARGS
 
@@ -270,7 +281,7 @@ __global__ void k_prepare_batch(const int* starts, const int* targets, int n, in
 // map's largest landmark distance, so that no pass over the estimates has to
 // find their maximum first.  With a search slot for every request the order is
 // of no use: they are copied.
-__global__ void __launch_bounds__(256) k_order_keys(const int4* req_in, const int* req_count, int4* req_out, int2* keys,
+__global__ void __launch_bounds__(128) k_order_keys(const int4* req_in, const int* req_count, int4* req_out, int2* keys,
                                                     int* hist, const unsigned short* lm, int L, int n, int lm_max,
                                                     int slots) {
     const int R = *req_count;
@@ -294,15 +305,19 @@ __global__ void __launch_bounds__(256) k_order_keys(const int4* req_in, const in
     }
 }
 
-__global__ void __launch_bounds__(1024) k_order_place(const int4* req_in, const int* req_count, int4* req_out,
-                                                      const int2* keys, const int* hist, int slots) {
+__global__ void __launch_bounds__(256) k_order_place(const int4* req_in, const int* req_count, int4* req_out,
+                                                     const int2* keys, const int* hist, int slots) {
     __shared__ int warp_tot[32];
-    __shared__ int start[kOrderBuckets];
+    __shared__ int4 start4[kOrderBuckets / 4];
+    static_assert(kOrderBuckets == 4 * 256, "four buckets per thread");
+    const int* start = reinterpret_cast<const int*>(start4);
     const int R = *req_count;
     if (R <= slots) return;
-    const int h = hist[threadIdx.x];
+    const int4 h = reinterpret_cast<const int4*>(hist)[threadIdx.x];
+    const int four = h.x + h.y + h.z + h.w;
     int tot;
-    start[threadIdx.x] = block_scan(h, warp_tot, &tot) - h;
+    const int before = block_scan<256>(four, warp_tot, &tot) - four;
+    start4[threadIdx.x] = make_int4(before, before + h.x, before + h.x + h.y, before + h.x + h.y + h.z);
     __syncthreads();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < R; i += gridDim.x * blockDim.x) {
         const int2 k = keys[i];
@@ -794,13 +809,14 @@ inline int blocks_for(int n, int bt) { return (n + bt - 1) / bt; }
 
 void launch_compact(cudaStream_t s, int A, int* state, const int* cur, const int* targ, int P,
                     const CompactScenes& scn, int4* req, int* req_count, unsigned char* in_move, int* mv_count,
-                    int* parity, int* work_ctr, int* hist, unsigned long long* stats, const FrameWords& words) {
-    if (A <= kCompactThreads * kCompactRun)
-        k_compact<<<1, kCompactThreads, 0, s>>>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count,
-                                                parity, work_ctr, hist, stats, words);
-    else
-        k_compact_cluster<<<kCompactCluster, kCompactThreads, 0, s>>>(A, state, cur, targ, P, scn, req, req_count,
-                                                                      in_move, mv_count, parity, work_ctr, hist, stats, words);
+                    int* parity, int* work_ctr, int* hist, unsigned long long* stats, const FrameWords& words,
+                    bool beside_searches) {
+    const int threads = beside_searches ? kBesideThreads : kCompactThreads;
+    const bool one = A <= threads * kCompactRun;
+    auto kernel = beside_searches ? (one ? k_compact<kBesideThreads> : k_compact_cluster<kBesideThreads>)
+                                  : (one ? k_compact<kCompactThreads> : k_compact_cluster<kCompactThreads>);
+    kernel<<<one ? 1 : kCompactCluster, threads, 0, s>>>(A, state, cur, targ, P, scn, req, req_count, in_move, mv_count,
+                                                         parity, work_ctr, hist, stats, words);
 }
 
 void launch_apply_targets(cudaStream_t s, const int4* recs, int n, int* state, int* targ_node,
@@ -835,9 +851,8 @@ void launch_edge_rows(cudaStream_t s, const SearchRow* rows, int n, EdgeRow* out
 void launch_order_requests(cudaStream_t s, const int4* req_in, const int* req_count, int most, int4* req_out,
                            const OrderParams& o, int n, int slots) {
     const int blocks = std::max(1, std::min(128, blocks_for(most, 256)));
-    k_order_keys<<<blocks, 256, 0, s>>>(req_in, req_count, req_out, o.keys, o.hist, o.lm, o.L, n, o.lm_max, slots);
-    k_order_place<<<std::min(32, blocks_for(most, 1024)), 1024, 0, s>>>(req_in, req_count, req_out, o.keys, o.hist,
-                                                                       slots);
+    k_order_keys<<<2 * blocks, 128, 0, s>>>(req_in, req_count, req_out, o.keys, o.hist, o.lm, o.L, n, o.lm_max, slots);
+    k_order_place<<<blocks, 256, 0, s>>>(req_in, req_count, req_out, o.keys, o.hist, slots);
 }
 
 void launch_move_bin(cudaStream_t s, const MoverParams& p) {

@@ -414,6 +414,7 @@ int serve_start(Context& c, int max_in_flight, std::string& err) {
     if (c.serve) return GMAPF_OK;
     Device& d = c.dev;
     SCK(cudaSetDevice(d.device));
+    device_drop_graph(c);  // (the frames' compaction is another while serving)
     Service* psv = new Service();
     c.serve = psv;
     Service& sv = *psv;
@@ -504,6 +505,7 @@ int serve_start(Context& c, int max_in_flight, std::string& err) {
 
 void serve_free(Context& c) {
     if (!c.serve) return;
+    device_drop_graph(c);
     Service& sv = *c.serve;
     for (int k = 0; k < kStreams; k++)
         if (sv.st[k]) cudaStreamSynchronize(sv.st[k]);

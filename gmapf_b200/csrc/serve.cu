@@ -373,34 +373,45 @@ int admit_and_launch(Context& c, Service& sv, std::string& err) {
             return GMAPF_E_DEVICE;
         }
     }
-    // the queries admitted since the last launch: one batch on an idle stream;
-    // more of them than a stream has slots go in equal parts to several, two of
-    // the idle ones left for later arrivals (4,096 queries at once between
-    // rectangles, T=8: one stream 339 us, six 75 us)
+    // The queries admitted since the last launch, as one batch on an idle stream.  More
+    // of them than a stream has slots take those of idle neighbours too, two idle
+    // streams left for later arrivals (4,096 queries at once between rectangles, T=8:
+    // one stream's slots 339 us, six streams' 75 us).  One launch: as one launch per
+    // stream they also kept the streams of the frames waiting, by whatever hardware
+    // queues the streams share (16,384 agents on the 64x64 maze, T=8: the next
+    // frame took 5.3 ms, the batch's time; now 0.15).
     if (sv.launched < sv.tail) {
-        int idle[kStreams], n_idle = 0;
-        for (int j = 0; j < kStreams; j++)
-            if (!sv.st_busy[j]) idle[n_idle++] = j;
+        int n_idle = 0, first = 0, run = 0;  // the first of the longest runs of idle streams
+        for (int j = 0, len = 0; j < kStreams; j++) {
+            n_idle += !sv.st_busy[j];
+            len = sv.st_busy[j] ? 0 : len + 1;
+            if (len > run) {
+                run = len;
+                first = j + 1 - len;
+            }
+        }
         const long long cnt = sv.tail - sv.launched;
         const long long want = (cnt + sv.slots_per_stream - 1) / sv.slots_per_stream;
-        const int parts = (int)std::min<long long>(want, n_idle > 3 ? n_idle - 2 : std::min(n_idle, 1));
-        for (int q = 0; q < parts; q++) {
-            const int k = idle[q];
-            const long long part = (sv.tail - sv.launched) / (parts - q);
-            sv.h_cnt[k] = (int)part;
+        const int parts = (int)std::min<long long>({want, n_idle > 3 ? n_idle - 2 : std::min(n_idle, 1), run});
+        if (parts > 0) {
+            const int k = first;
+            sv.h_cnt[k] = (int)cnt;
             cudaStream_t st = sv.st[k];
             if (sv.copy_recorded) SCK(cudaStreamWaitEvent(st, sv.copied, 0));
             SCK(cudaMemsetAsync(sv.d_wc + 2 * k, 0, sizeof(int), st));
             SCK(cudaMemcpyAsync(sv.d_wc + 2 * k + 1, sv.h_cnt + k, sizeof(int), cudaMemcpyHostToDevice, st));
             SearchParams sp = serve_params(c, sv, k);
+            sp.slots = parts * sv.slots_per_stream;
             const int gpb = c.block_threads / 32;
-            const long long warps = std::min<long long>(part, sv.slots_per_stream);
+            const long long warps = std::min<long long>(cnt, sp.slots);
             const int blocks = (int)((warps + gpb - 1) / gpb);
             SCK(launch_search(st, sp, blocks, c.block_threads, true, 0, c.dev.vm, c.dev.bm_words));
             SCK(cudaMemcpyAsync(sv.h_err + k, sv.d_err + k, sizeof(int), cudaMemcpyDeviceToHost, st));
-            SCK(cudaEventRecord(sv.st_done[k], st));
-            sv.st_busy[k] = true;
-            sv.launched += part;
+            for (int j = k; j < k + parts; j++) {
+                SCK(cudaEventRecord(sv.st_done[j], st));
+                sv.st_busy[j] = true;
+            }
+            sv.launched = sv.tail;
             sv.launches++;
             c.launches++;
         }

@@ -1,11 +1,41 @@
-"""Frames of a serving context: their compaction (made of smaller blocks while
-serving) gives the requests of any other frame."""
+"""Frames of a serving context: they do not wait for the searches in flight, and
+their compaction (made of smaller blocks while serving) is the frames' own."""
 import numpy as np
 import pytest
 
 import gmapf_b200 as G
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,Cap", [(8, 32), (32, 16)])
+@pytest.mark.parametrize("A", [3000, 6000])
+def test_frame_beside_long_searches(A, T, Cap):
+    # every agent is sent from one end of a corridor of 20,000 triangles to the
+    # other: some ten thousand rounds each (milliseconds), and a frame of a fraction
+    # of one is over before the first search is
+    from test_gpu_frame_kernels import inside, winding_map
+    nodes = winding_map(100, 100, 8.0)
+    rng = np.random.default_rng(A)
+    g = G.GMAPF()
+    g.Init(G.make_config(A, 0.1, 1.0, A, T, Cap))
+    g.FillMapManually(nodes)
+    for p in inside(nodes[:200], A, rng):
+        g.AddAgent(p)
+    g.serve_start(A)
+    ids = np.arange(A, dtype=np.int32)
+    g.serve_submit(ids[:8], inside(nodes[:200], 8, rng))
+    g.serve_drain()
+    g.AsyncStep(1.0)  # the first frame records its graph
+    g.WaitStepEnd()
+    g.serve_submit(ids, inside(nodes[-200:], A, rng))
+    g.AsyncStep(1.0)
+    g.WaitStepEnd()
+    g.serve_poll()
+    done = g.serve_stats()["completed"] - 8
+    g.serve_drain()
+    assert done == 0
+    assert g.serve_stats()["found"] == A + 8
 
 
 @pytest.mark.parametrize("A", [3, 1023, 1024, 1025, 8192, 8195, 16390])

@@ -207,8 +207,9 @@ MoverParams mover_params(Context& c) {
     p.cells = d.cells;
     p.cell_of = d.cell_of;
     p.parity = d.counters + CT_PARITY;
-    p.cell_head = d.cell_head;
+    p.cell_count = d.cell_count;
     p.bucket = d.bucket;
+    p.lists = d.lists;
     p.next = d.next;
     p.tri = d.tri;
     p.cen = d.cen;
@@ -650,8 +651,9 @@ int device_start(Context& c, std::string& err) {
         CK(cudaMemcpy(d.scene_P, sp.data(), sizeof(int) * sp.size(), cudaMemcpyHostToDevice));
     }
     DALLOC(d.cell_of, A);
-    DALLOC(d.cell_head, 2 * (size_t)d.cells);
+    DALLOC(d.cell_count, 2 * (size_t)d.cells);
     DALLOC(d.bucket, 4 * (size_t)d.cells);
+    DALLOC(d.lists, 4 * (size_t)d.cells);
     DALLOC(d.next, A);
 
     // pinned host staging

@@ -157,9 +157,10 @@ struct MoverParams {
     // agent grid (all scenes' cells, global ids)
     int cells;
     int* cell_of;
-    int* parity;       // [0] whose turn of the two copies of cell_head it is, [1] the copy has been used
-    int2* cell_head;   // 2 x cells: agents in the cell, list of those beyond its bucket
+    int* parity;       // [0] whose turn of the two copies of cell_count it is, [1] the copy has been used
+    int* cell_count;   // 2 x cells: agents in the cell
     int* bucket;       // 4 x cells: the first agents of a cell
+    int* lists;        // 4 x cells: the last agents of the lists of those beyond its bucket
     int* next;         // A: the lists
     // map
     const float2* tri; // 3 vertices per triangle, global ids
@@ -372,8 +373,7 @@ struct Device {
     int bm_words = 0;           // bitmap words per slot
     int rec_cap = 0, log_cap = 0, gbm_cap = 0;  // slots the records / logs / bitmaps hold (kept across reshapes)
     // agent grid
-    int *cell_of = nullptr, *bucket = nullptr, *next = nullptr;
-    int2* cell_head = nullptr;
+    int *cell_of = nullptr, *cell_count = nullptr, *bucket = nullptr, *lists = nullptr, *next = nullptr;
     int cells = 0;
     // scenes (ScenePar per scene; the rest only when there is more than one)
     ScenePar* scene_par = nullptr;

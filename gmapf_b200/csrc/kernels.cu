@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(256) k_order_place(const int4* req_in, const i
 }
 
 // The agent grid of a frame: per cell a count and, for the agents beyond the
-// four of its bucket, the head of a list (agent + 1, 0: none).  Cells hold about
+// four of its bucket, four lists that they join in turn.  Cells hold about
 // one agent on average (5% of the agents of a uniform crowd find their bucket
 // full), so one 16-byte read gives a cell's agents, and binning is one pass: no
 // scan over the cells and no second pass to place the agents (k_cell_scan and
@@ -334,15 +334,22 @@ __global__ void __launch_bounds__(256) k_order_place(const int4* req_in, const i
 // Two copies of the counts take turns, so that a frame's binning clears the
 // other frame's without a launch of its own; *p.parity says whose turn it is (the
 // compaction switches it once the collision pass has marked the copy as used).
-constexpr int kBucket = 4;
+// The buckets and the lists' heads are not cleared: the count says how many
+// entries each holds.
+//
+// Where a crowd gathers a cell holds hundreds.  Its four lists are followed
+// together, as each step of a list waits for the one before: the mover of 4,096
+// agents within 118 units of one place (2,000 agents in the nine cells of each) takes
+// 3.4 ms, with one list per cell 4.5, with the cells' agents sorted into runs 4.0.
+constexpr int kBucket = 4, kLists = 4;
 
 // move (AgentsMover.h:51-71) fused with the binning
 __global__ void k_move_bin(MoverParams p) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (*p.mv_count == 0) return;  // AgentsMover.h:296-297
     const int turn = *p.parity & 1;
-    int2* const old = p.cell_head + (size_t)(1 - turn) * p.cells;
-    for (int k = i; k < p.cells; k += gridDim.x * blockDim.x) old[k] = make_int2(0, 0);
+    int* const old = p.cell_count + (size_t)(1 - turn) * p.cells;
+    for (int k = i; k < p.cells; k += gridDim.x * blockDim.x) old[k] = 0;
     if (i >= p.A) return;
     const ScenePar& sc = p.sc[p.agent_scene ? p.agent_scene[i] : 0];
     float2 c = p.pos[i];
@@ -364,14 +371,38 @@ __global__ void k_move_bin(MoverParams p) {
         const int cx = grid_cell(c.x, sc.ax0, sc.ainv, sc.aw);
         const int cy = grid_cell(c.y, sc.ay0, sc.ainv, sc.ah);
         cell = sc.cell_base + cy * sc.aw + cx;
-        int2* const h = p.cell_head + (size_t)turn * p.cells + cell;
-        const int k = atomicAdd(&h->x, 1);
+        const int k = atomicAdd(p.cell_count + (size_t)turn * p.cells + cell, 1);
         if (k < kBucket)
             p.bucket[kBucket * (size_t)cell + k] = i;
-        else
-            p.next[i] = atomicExch(&h->y, i + 1);
+        else  // (the first of a list takes what an earlier frame left as its next, which is never followed)
+            p.next[i] = atomicExch(p.lists + kLists * (size_t)cell + (k & (kLists - 1)), i);
     }
     p.cell_of[i] = cell;
+}
+
+// f(agent, its position) for the first min(n, 4) of q
+template <class F>
+__device__ __forceinline__ void each_of(const MoverParams& p, int4 q, int n, const F& f) {
+    const int j[4] = {q.x, q.y, q.z, q.w};
+    float2 o[4];
+#pragma unroll
+    for (int m = 0; m < 4; m++) o[m] = m < n ? p.pos_mid[j[m]] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+        if (m < n) f(j[m], o[m]);
+}
+
+// the same for the `n` agents of a cell beyond its bucket: list m holds those
+// numbered m, m + 4, ... of them (a step reads no further than its list goes)
+template <class F>
+__device__ __forceinline__ void each_beyond(const MoverParams& p, int cell, int n, const F& f) {
+    int4 q = *reinterpret_cast<const int4*>(p.lists + kLists * (size_t)cell);
+    for (; n > 0; n -= kLists) {
+        const int4 r = make_int4(n > 4 ? p.next[q.x] : 0, n > 5 ? p.next[q.y] : 0, n > 6 ? p.next[q.z] : 0,
+                                 n > 7 ? p.next[q.w] : 0);
+        each_of(p, q, n, f);
+        q = r;
+    }
 }
 
 constexpr int kMaxLocal = 16;
@@ -425,7 +456,7 @@ __global__ void __launch_bounds__(64, 8) k_collide_progress(MoverParams p) {
     int si = p.step_idx[i];
     const int sn = p.step_node[i];
     const float2 step_pos = p.step_pos[i];
-    const int2* const heads = p.cell_head + (size_t)(*p.parity & 1) * p.cells;
+    const int* const counts = p.cell_count + (size_t)(*p.parity & 1) * p.cells;
     float2 tri[3];  // the step's triangle
     if (moving && sn >= 0 && sn < p.n) {
 #pragma unroll
@@ -436,26 +467,26 @@ __global__ void __launch_bounds__(64, 8) k_collide_progress(MoverParams p) {
     if (c >= 0) {
         const int lc = c - sc.cell_base;  // cell within the agent's scene
         const int cx = lc % sc.aw, cy = lc / sc.aw;
-        int2 h[9];
+        int h[9];
         int4 b[9];
         unsigned over = 0;  // cells with agents beyond their bucket
 #pragma unroll
         for (int k = 0; k < 9; k++) {
             const int x = cx + k % 3 - 1, y = cy + k / 3 - 1;
             const bool in = x >= 0 && x < sc.aw && y >= 0 && y < sc.ah;
-            h[k] = in ? heads[sc.cell_base + y * sc.aw + x] : make_int2(0, 0);
+            h[k] = in ? counts[sc.cell_base + y * sc.aw + x] : 0;
         }
 #pragma unroll
         for (int k = 0; k < 9; k++) {
-            examined += h[k].x;
-            over |= (h[k].y != 0 ? 1u : 0u) << k;
+            examined += h[k];
+            over |= (h[k] > kBucket ? 1u : 0u) << k;
             b[k] = make_int4(-1, -1, -1, -1);
-            if (h[k].x > 0)
+            if (h[k] > 0)
                 b[k] = *reinterpret_cast<const int4*>(p.bucket + kBucket * (size_t)(c + (k / 3 - 1) * sc.aw + k % 3 - 1));
             // (entries beyond the count are a former frame's)
-            if (h[k].x < 2) b[k].y = -1;
-            if (h[k].x < 3) b[k].z = -1;
-            if (h[k].x < 4) b[k].w = -1;
+            if (h[k] < 2) b[k].y = -1;
+            if (h[k] < 3) b[k].z = -1;
+            if (h[k] < 4) b[k].w = -1;
         }
         Pushes ps;
         auto meet = [&](int j, float2 o) {
@@ -485,10 +516,10 @@ __global__ void __launch_bounds__(64, 8) k_collide_progress(MoverParams p) {
         }
         for (; over; over &= over - 1) {
             const int k = __ffs(over) - 1;
-            const int2 q = heads[c + (k / 3 - 1) * sc.aw + k % 3 - 1];
-            int left = q.x - kBucket;  // (the count bounds the walk)
-            for (int j = q.y - 1; j >= 0 && left > 0; j = p.next[j] - 1, left--)
-                if (j != i) meet(j, p.pos_mid[j]);
+            const int cell = c + (k / 3 - 1) * sc.aw + k % 3 - 1;
+            each_beyond(p, cell, counts[cell] - kBucket, [&](int j, float2 o) {
+                if (j != i) meet(j, o);
+            });
         }
         float sx = 0.f, sy = 0.f;
         int total = 0;
@@ -504,9 +535,8 @@ __global__ void __launch_bounds__(64, 8) k_collide_progress(MoverParams p) {
             for (;;) {
                 int best = 0x7fffffff;
                 float bvx = 0.f, bvy = 0.f;
-                auto look = [&](int j) {
+                auto look = [&](int j, float2 o) {
                     if (j == i || j <= last || j >= best) return;
-                    const float2 o = p.pos_mid[j];
                     const float dx = GM_FSUB(me.x, o.x), dy = GM_FSUB(me.y, o.y);
                     const float d2 = GM_FADD(GM_FMUL(dx, dx), GM_FMUL(dy, dy));
                     if (!(d2 < sc.cd2)) return;
@@ -519,10 +549,9 @@ __global__ void __launch_bounds__(64, 8) k_collide_progress(MoverParams p) {
                 for (int y = max(cy - 1, 0); y <= min(cy + 1, sc.ah - 1); y++)
                     for (int x = max(cx - 1, 0); x <= min(cx + 1, sc.aw - 1); x++) {
                         const int cc = sc.cell_base + y * sc.aw + x;
-                        const int2 q = heads[cc];
-                        for (int k = 0; k < min(q.x, kBucket); k++) look(p.bucket[kBucket * (size_t)cc + k]);
-                        int left = q.x - kBucket;
-                        for (int j = q.y - 1; j >= 0 && left > 0; j = p.next[j] - 1, left--) look(j);
+                        const int n = counts[cc];
+                        if (n > 0) each_of(p, *reinterpret_cast<const int4*>(p.bucket + kBucket * (size_t)cc), n, look);
+                        if (n > kBucket) each_beyond(p, cc, n - kBucket, look);
                     }
                 if (best == 0x7fffffff) break;
                 sx = GM_FADD(sx, bvx);

@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
                     p.ag_state[agent] = GMAPF_AGENT_IDLE;
                     p.ag_path_len[agent] = 0;
                 }
-                if (!bad) atomicAdd(p.stats + ST_FOUND, 1ull);
+                if (!bad && p.stats) atomicAdd(p.stats + ST_FOUND, 1ull);
                 if (p.done) ring_complete(p, orow, p.ring_base + r, bad ? 0 : 1);
             }
             continue;
@@ -935,12 +935,14 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
                 if (found) p.ag_step_idx[agent] = -1;
                 p.ag_path_len[agent] = L;
             }
-            atomicAdd(p.stats + ST_EXPANSIONS, (unsigned long long)expansions);
-            atomicAdd(p.stats + ST_DEG_SUM, (unsigned long long)ds);
-            atomicAdd(p.stats + ST_ROUNDS, (unsigned long long)rounds);
-            atomicAdd(p.stats + ST_CLAIMS, (unsigned long long)claims);
-            atomicAdd(p.stats + ST_PATH_NODES, (unsigned long long)L);
-            atomicAdd(p.stats + ST_FOUND, (unsigned long long)found);
+            if (p.stats) {
+                atomicAdd(p.stats + ST_EXPANSIONS, (unsigned long long)expansions);
+                atomicAdd(p.stats + ST_DEG_SUM, (unsigned long long)ds);
+                atomicAdd(p.stats + ST_ROUNDS, (unsigned long long)rounds);
+                atomicAdd(p.stats + ST_CLAIMS, (unsigned long long)claims);
+                atomicAdd(p.stats + ST_PATH_NODES, (unsigned long long)L);
+                atomicAdd(p.stats + ST_FOUND, (unsigned long long)found);
+            }
             if (p.done) ring_complete(p, orow, p.ring_base + r, found);
             if (p.timeline) p.timeline[2 * (long long)orow + 1] = global_timer_ns();
         }

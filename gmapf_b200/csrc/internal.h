@@ -99,7 +99,7 @@ struct SearchParams {
     int* ag_state;           // agent arrays (step) or null
     int* ag_step_idx;
     int* ag_path_len;
-    unsigned long long* stats;  // ST_COUNT counters
+    unsigned long long* stats;  // ST_COUNT counters (null: none are kept, corridor.cu's placement 1 only)
     int* err;
     // search state slots [slot_base, slot_base + slots) of rec/epoch/log/queues/gbm
     int slot_base;

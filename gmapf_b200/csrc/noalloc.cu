@@ -47,8 +47,8 @@ constexpr size_t kHeaderBytes = 256;
 constexpr int kMaxDevices = 64;
 
 // header: 32-bit work counter at byte 0, 64-bit query counter at byte 8, error
-// bits at 16 and counters from 64 (written, not read: results carry the codes)
-constexpr size_t kWorkOff = 0, kQueryOff = 8, kErrOff = 16, kStatsOff = 64;
+// bits at 16 (written, not read: results carry the codes)
+constexpr size_t kWorkOff = 0, kQueryOff = 8, kErrOff = 16;
 
 // Query stamps of the record form start here.  The log form leaves edge rows,
 // centroids and log entries in the same array; the upper word of a stamp, read
@@ -376,8 +376,9 @@ __device__ __forceinline__ int leading(const gmapf_node& nd) {
     return deg;
 }
 
-__global__ void k_noalloc_rows(const gmapf_node* nodes, int n, EdgeRow* rows, EdgeHalf* third, float2* cen) {
+__global__ void k_noalloc_rows(const gmapf_node* nodes, int n, EdgeRow* rows, EdgeHalf* third, float2* cen, int* work) {
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == 0) *work = 0;  // the call's work counter
     if (k >= 4ll * n) return;
     const int v = (int)(k >> 2), s = (int)(k & 3);
     const gmapf_node& nd = nodes[v];
@@ -553,11 +554,6 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
     if (slots < 1) slots = 1;
     const int blocks = (int)slots;
 
-    // the work counter must start at zero for every call
-    if (cudaMemsetAsync(ds->scratch + kWorkOff, 0, sizeof(unsigned), s) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(GMAPF_E_CUDA, "clearing the work counter failed");
-    }
     NoAllocArgs a;
     a.nodes = d_nodes;
     a.n = n_nodes;
@@ -586,7 +582,7 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
         const long long per_sm_log = std::max<long long>(1, std::min<long long>(24, 228 * 1024 / (long long)(smem + 1024)));
         const int blocks_log = (int)std::min({lay.slots, per_sm_log * ds->sms, (long long)n_queries});
         k_noalloc_rows<<<(unsigned)((4ll * n_nodes + 255) / 256), 256, 0, s>>>(d_nodes, n_nodes, lay.rows, lay.third,
-                                                                              lay.cen);
+                                                                              lay.cen, reinterpret_cast<int*>(ds->scratch + kWorkOff));
         SearchParams p{};
         p.erow = lay.rows;
         p.third = lay.third;
@@ -607,13 +603,17 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
         p.path_stride = path_stride;
         p.out_found = d_found;
         p.out_len = d_lens;
-        p.stats = reinterpret_cast<unsigned long long*>(ds->scratch + kStatsOff);
         p.err = reinterpret_cast<int*>(ds->scratch + kErrOff);
         p.bad_code = -1;
         p.cut_code = -2;
         e = launch_corridor_search(s, p, blocks_log, 32, true, 0, 1, bm_words);
         if (e != cudaSuccess) return fail(GMAPF_E_CUDA, cudaGetErrorString(e));
         return GMAPF_OK;
+    }
+    // the work counter must start at zero for every call (the log form's rows kernel does it)
+    if (cudaMemsetAsync(ds->scratch + kWorkOff, 0, sizeof(unsigned), s) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(GMAPF_E_CUDA, "clearing the work counter failed");
     }
     switch (T) {
         case 2: e = run_t<2>(a, blocks, s); break;

@@ -46,9 +46,25 @@ constexpr size_t kScratchBytes = size_t(64) << 20;  // 64 MiB per device
 constexpr size_t kHeaderBytes = 256;
 constexpr int kMaxDevices = 64;
 
-// header: 32-bit work counter at byte 0, 64-bit query counter at byte 8, error
-// bits at 16 (written, not read: results carry the codes)
-constexpr size_t kWorkOff = 0, kQueryOff = 8, kErrOff = 16;
+// header: 32-bit work counter at byte 0, queries left for the log form at 4, 64-bit
+// query counter at 8, error bits at 16 (written, not read: results carry the codes)
+constexpr size_t kWorkOff = 0, kLeftOff = 4, kQueryOff = 8, kErrOff = 16;
+
+// Few queries on a large navmesh: the log form lays out the whole navmesh first
+// (152 bytes per triangle), the record form touches what it searches.  From
+// kLargeNavmesh triangles on, a call with a record slot for every query (T <= 8: two
+// queries per slot) runs the record form for short_rounds(T) rounds, and only queries
+// that need more are left to the log form.  One query to a triangle a few steps away
+// at T=8, then with the log form alone, then with the records alone: 146,000
+// triangles 34, 49, 23 us, 289,000 30, 49, 22 us, 387,000 27, 53, 21 us; one across the
+// 147,000-triangle maze 13.0, 13.6, 32.9 ms.  On smaller navmeshes the layout costs 6 to
+// 13 us and the two launches more after a short record form 8.
+constexpr int kLargeNavmesh = 1 << 17;
+constexpr int short_rounds(int T) { return T <= 8 ? 16 : 8; }
+// (the queries left are listed at the array's end)
+constexpr size_t kLeftBytes = 1024;
+static_assert(kLeftBytes / sizeof(int4) >= 2 * (kScratchBytes / (size_t(kLargeNavmesh) * 32)),
+              "the list holds two queries per record slot");
 
 // Query stamps of the record form start here.  The log form leaves edge rows,
 // centroids and log entries in the same array; the upper word of a stamp, read
@@ -127,6 +143,8 @@ struct NoAllocArgs {
     long long stride;
     unsigned char* scratch;  // device address of g_scratch
     int slots;
+    int short_rounds;  // a search still running after them is left to the log form (0: none is)
+    int4* left;        // those: {-1, start, target, query}, counted at kLeftOff
 };
 
 // One warp per request; the same rounds, claim order and queue rules as the
@@ -187,7 +205,7 @@ __global__ void __launch_bounds__(32) k_search_noalloc(NoAllocArgs a) {
         }
         __syncwarp();
         int found = 0, mS = 0, gS = 0, mT = 0, gT = 0, rounds = 0;
-        bool capped = false;
+        bool capped = false, later = false;
         for (;;) {
             rounds++;
             int idu = -1, gdu = 0, uk = 0;
@@ -313,6 +331,10 @@ __global__ void __launch_bounds__(32) k_search_noalloc(NoAllocArgs a) {
                     ended = true;
                     capped = true;
                 }
+                if (!ended && rounds == a.short_rounds) {
+                    ended = true;
+                    later = true;
+                }
             }
             __syncwarp();
             if (ended) break;
@@ -349,7 +371,9 @@ __global__ void __launch_bounds__(32) k_search_noalloc(NoAllocArgs a) {
             }
         }
         __syncwarp();
-        if (lane == 0) {
+        if (lane == 0 && later) {
+            a.left[atomicAdd(reinterpret_cast<int*>(a.scratch + kLeftOff), 1)] = make_int4(-1, start, target, r);
+        } else if (lane == 0) {
             a.found[r] = capped ? -2 : found;
             a.lens[r] = L;  // a length above path_stride means the row was left unwritten
         }
@@ -376,41 +400,45 @@ __device__ __forceinline__ int leading(const gmapf_node& nd) {
     return deg;
 }
 
-__global__ void k_noalloc_rows(const gmapf_node* nodes, int n, EdgeRow* rows, EdgeHalf* third, float2* cen, int* work) {
-    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k == 0) *work = 0;  // the call's work counter
-    if (k >= 4ll * n) return;
-    const int v = (int)(k >> 2), s = (int)(k & 3);
-    const gmapf_node& nd = nodes[v];
-    const int deg = leading(nd);
-    const int parent = s < deg ? nd.NeibsIdx[s] : -1;
-    EdgeRow o{{-1, (unsigned)deg << 4, 0.f, 0.f}, {-1, 0, 0.f, 0.f}};
-    EdgeHalf z{-1, 0, 0.f, 0.f};
-    int found = 0;
-    for (int j = 0; j < deg; j++) {
-        const int w = nd.NeibsIdx[j];
-        if (w == parent || w < 0 || w >= n) continue;
-        const gmapf_node& q = nodes[w];
-        int back = 3;
-        for (int b = leading(q) - 1; b >= 0; b--)
-            if (q.NeibsIdx[b] == v) back = b;
-        const float2 c = node_centroid(nodes, w);
-        if (found < 2) {
-            EdgeHalf& h = found == 0 ? o.x : o.y;
-            h.e = w << 2 | back;
-            h.info |= 1u << j;
-            h.x = c.x;
-            h.y = c.y;
-        } else {
-            z = EdgeHalf{w << 2 | back, 1u << j, c.x, c.y};
-            o.x.info |= kEdgeThird;
+// (left: null, or how many queries need the rows)
+__global__ void __launch_bounds__(256) k_noalloc_rows(const gmapf_node* nodes, int n, EdgeRow* rows, EdgeHalf* third,
+                                                      float2* cen, int* work, const int* left) {
+    const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (first == 0) *work = 0;  // the log form's work counter
+    if (left && *left == 0) return;
+    for (long long k = first; k < 4ll * n; k += (long long)gridDim.x * blockDim.x) {
+        const int v = (int)(k >> 2), s = (int)(k & 3);
+        const gmapf_node& nd = nodes[v];
+        const int deg = leading(nd);
+        const int parent = s < deg ? nd.NeibsIdx[s] : -1;
+        EdgeRow o{{-1, (unsigned)deg << 4, 0.f, 0.f}, {-1, 0, 0.f, 0.f}};
+        EdgeHalf z{-1, 0, 0.f, 0.f};
+        int found = 0;
+        for (int j = 0; j < deg; j++) {
+            const int w = nd.NeibsIdx[j];
+            if (w == parent || w < 0 || w >= n) continue;
+            const gmapf_node& q = nodes[w];
+            int back = 3;
+            for (int b = leading(q) - 1; b >= 0; b--)
+                if (q.NeibsIdx[b] == v) back = b;
+            const float2 c = node_centroid(nodes, w);
+            if (found < 2) {
+                EdgeHalf& h = found == 0 ? o.x : o.y;
+                h.e = w << 2 | back;
+                h.info |= 1u << j;
+                h.x = c.x;
+                h.y = c.y;
+            } else {
+                z = EdgeHalf{w << 2 | back, 1u << j, c.x, c.y};
+                o.x.info |= kEdgeThird;
+            }
+            found++;
         }
-        found++;
-    }
-    rows[k] = o;
-    if (s == 3) {
-        third[v] = z;
-        cen[v] = node_centroid(nodes, v);
+        rows[k] = o;
+        if (s == 3) {
+            third[v] = z;
+            cen[v] = node_centroid(nodes, v);
+        }
     }
 }
 
@@ -428,7 +456,8 @@ LogLayout log_layout(unsigned char* scratch, int n) {
                  cen = up(third + sizeof(EdgeHalf) * (size_t)n), logs = up(cen + sizeof(float2) * (size_t)n);
     LogLayout l{reinterpret_cast<EdgeRow*>(scratch + rows), reinterpret_cast<EdgeHalf*>(scratch + third),
                 reinterpret_cast<float2*>(scratch + cen), scratch + logs, n <= kPackedLogNodes ? 6 : 8, 0};
-    if (logs < kScratchBytes) l.slots = (long long)((kScratchBytes - logs) / (l.entry * (size_t)n));
+    const size_t end = kScratchBytes - (n >= kLargeNavmesh ? kLeftBytes : 0);
+    if (logs < end) l.slots = (long long)((end - logs) / (l.entry * (size_t)n));
     return l;
 }
 
@@ -552,7 +581,6 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
     slots = std::min(slots, by_mem);
     slots = std::min(slots, (long long)n_queries);
     if (slots < 1) slots = 1;
-    const int blocks = (int)slots;
 
     NoAllocArgs a;
     a.nodes = d_nodes;
@@ -572,32 +600,68 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
     a.stride = path_stride;
     a.scratch = ds->scratch;
     a.slots = (int)slots;
+    a.short_rounds = 0;
+    a.left = reinterpret_cast<int4*>(ds->scratch + kScratchBytes - kLeftBytes);
     cudaError_t e;
+    int* const work = reinterpret_cast<int*>(ds->scratch + kWorkOff);
+    int* const left = reinterpret_cast<int*>(ds->scratch + kLeftOff);
+    auto run_records = [&]() -> cudaError_t {
+        // the work counter must start at zero for every call (the log form's rows
+        // kernel clears it too), and no query is left yet
+        static_assert(kLeftOff == kWorkOff + sizeof(int), "cleared together");
+        const cudaError_t ce = cudaMemsetAsync(work, 0, 2 * sizeof(int), s);
+        if (ce != cudaSuccess) return ce;
+        switch (T) {
+            case 2: return run_t<2>(a, a.slots, s);
+            case 4: return run_t<4>(a, a.slots, s);
+            case 8: return run_t<8>(a, a.slots, s);
+            case 16: return run_t<16>(a, a.slots, s);
+            default: return run_t<32>(a, a.slots, s);
+        }
+    };
     // the log form, where its layout leaves as many slots as the record form has
     // (or one for every query) and a warp's share fits in shared memory
     const LogLayout lay = log_layout(ds->scratch, n_nodes);
     const int bm_words = search_bitmap_words(n_nodes);
     const size_t smem = corridor_smem_bytes(C, 32, bm_words, T, 1);
     if (lay.slots >= std::min(by_mem, (long long)n_queries) && smem <= 227 * 1024 && ds->log_ready[T]) {
+        // (the records leave the list its place)
+        const long long records =
+            (long long)((kScratchBytes - kHeaderBytes - kLeftBytes) / ((size_t)n_nodes * sizeof(NRec)));
+        const bool few = n_nodes >= kLargeNavmesh && n_queries <= (T <= 8 ? 2 : 1) * records;
+        if (few) {
+            if (a.max_rounds > short_rounds(T)) a.short_rounds = short_rounds(T);
+            a.slots = (int)std::min<long long>(a.slots, records);
+            e = run_records();
+            if (e != cudaSuccess) return fail(GMAPF_E_CUDA, cudaGetErrorString(e));
+            if (a.short_rounds == 0) return GMAPF_OK;
+        }
         const long long per_sm_log = std::max<long long>(1, std::min<long long>(24, 228 * 1024 / (long long)(smem + 1024)));
         const int blocks_log = (int)std::min({lay.slots, per_sm_log * ds->sms, (long long)n_queries});
-        k_noalloc_rows<<<(unsigned)((4ll * n_nodes + 255) / 256), 256, 0, s>>>(d_nodes, n_nodes, lay.rows, lay.third,
-                                                                              lay.cen, reinterpret_cast<int*>(ds->scratch + kWorkOff));
+        // (where no query may be left, few blocks that find that out)
+        const long long row_blocks = std::min<long long>((4ll * n_nodes + 255) / 256, few ? 8ll * ds->sms : 1ll << 30);
+        k_noalloc_rows<<<(unsigned)row_blocks, 256, 0, s>>>(d_nodes, n_nodes, lay.rows, lay.third, lay.cen, work,
+                                                            few ? left : nullptr);
         SearchParams p{};
         p.erow = lay.rows;
         p.third = lay.third;
         p.cen = lay.cen;
         p.n = n_nodes;
-        p.starts = d_starts;
-        p.targets = d_targets;
-        p.req_count_h = n_queries;
+        if (few) {
+            p.req = a.left;
+            p.req_count_d = left;
+        } else {
+            p.starts = d_starts;
+            p.targets = d_targets;
+            p.req_count_h = n_queries;
+        }
         p.T = T;
         p.C = C;
         p.K = heuristic_k;
         p.log = lay.logs;
         p.log_bytes = lay.entry;
         p.slots = blocks_log;
-        p.work_ctr = reinterpret_cast<int*>(ds->scratch + kWorkOff);
+        p.work_ctr = work;
         p.max_rounds = a.max_rounds;
         p.paths = d_paths;
         p.path_stride = path_stride;
@@ -610,18 +674,7 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
         if (e != cudaSuccess) return fail(GMAPF_E_CUDA, cudaGetErrorString(e));
         return GMAPF_OK;
     }
-    // the work counter must start at zero for every call (the log form's rows kernel does it)
-    if (cudaMemsetAsync(ds->scratch + kWorkOff, 0, sizeof(unsigned), s) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(GMAPF_E_CUDA, "clearing the work counter failed");
-    }
-    switch (T) {
-        case 2: e = run_t<2>(a, blocks, s); break;
-        case 4: e = run_t<4>(a, blocks, s); break;
-        case 8: e = run_t<8>(a, blocks, s); break;
-        case 16: e = run_t<16>(a, blocks, s); break;
-        default: e = run_t<32>(a, blocks, s); break;
-    }
+    e = run_records();
     if (e != cudaSuccess) return fail(GMAPF_E_CUDA, cudaGetErrorString(e));
     return GMAPF_OK;
 }

@@ -879,14 +879,8 @@ int device_wait_step(Context& c, std::string& err) {
     return GMAPF_OK;
 }
 
-int device_locate_points(Context& c, const gmapf_v2* pts, int n, int* node, std::string& err) {
+int device_reserve_locate(Context& c, int n, std::string& err) {
     Device& d = c.dev;
-    if (n <= 0) return GMAPF_OK;
-    if (c.scene_par.size() != 1) {
-        err = "device point location needs a single-map context";
-        return GMAPF_E_STATE;
-    }
-    CK(cudaSetDevice(d.device));
     if (!d.loc_stream) CK(cudaStreamCreateWithFlags(&d.loc_stream, cudaStreamNonBlocking));
     if (n > d.loc_cap) {
         cudaFree(d.loc_pts);
@@ -905,6 +899,19 @@ int device_locate_points(Context& c, const gmapf_v2* pts, int n, int* node, std:
         CK(cudaHostAlloc(&d.h_loc_node, sizeof(int) * cap, cudaHostAllocDefault));
         d.loc_cap = cap;
     }
+    return GMAPF_OK;
+}
+
+int device_locate_points(Context& c, const gmapf_v2* pts, int n, int* node, std::string& err) {
+    Device& d = c.dev;
+    if (n <= 0) return GMAPF_OK;
+    if (c.scene_par.size() != 1) {
+        err = "device point location needs a single-map context";
+        return GMAPF_E_STATE;
+    }
+    CK(cudaSetDevice(d.device));
+    const int rc = device_reserve_locate(c, n, err);
+    if (rc) return rc;
     static_assert(sizeof(gmapf_v2) == sizeof(float2), "point layout");
     std::memcpy(d.h_loc_pts, pts, sizeof(float2) * n);
     CK(cudaMemcpyAsync(d.loc_pts, d.h_loc_pts, sizeof(float2) * n, cudaMemcpyHostToDevice, d.loc_stream));

@@ -505,6 +505,8 @@ int device_upload_batch_io(Context& c, int n, long long path_stride, std::string
 // the triangle of each of n host points, located on the device with the
 // same rule as the host (single-map context, after start); blocks until done
 int device_locate_points(Context& c, const gmapf_v2* pts, int n, int* node, std::string& err);
+// its buffers for n points at a time (Device::loc_cap; a larger call replaces them, which waits for the GPU)
+int device_reserve_locate(Context& c, int n, std::string& err);
 int device_set_targets_device(Context& c, const int* d_ids, const gmapf_v2* d_pos, int n, int id_base,
                               int id_count, std::string& err);
 

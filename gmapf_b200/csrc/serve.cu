@@ -545,10 +545,24 @@ int serve_submit(Context& c, const int* ids, const gmapf_v2* pos, int n, const i
     std::vector<Waiting> batch(n);
     const long long now = now_ns();
     // A large burst's points are located on the device (targets, then the points
-    // under the agents; same rule): 8,192 points took 330 us here.
+    // under the agents; same rule): 8,192 points took 330 us here.  The buffers are made
+    // once, for all agents; while searches are in flight they are not replaced by
+    // larger ones, which would wait for those: more points go in portions.  Where the
+    // device does not answer, the points are located here.
     constexpr int kDeviceLocate = 1024;
     std::vector<int> node;
-    if (n >= kDeviceLocate && !c.is_world && sv.room) {
+    bool on_device = n >= kDeviceLocate && !c.is_world && sv.room;
+    if (on_device) {
+        SCK(cudaSetDevice(c.dev.device));
+        const int all = 2 * std::max(n, std::min(c.A, 1 << 20));
+        if (c.dev.loc_cap == 0 || (sv.pending == 0 && 2 * n > c.dev.loc_cap))
+            on_device = device_reserve_locate(c, all, err) == GMAPF_OK;
+        if (!on_device) {
+            cudaGetLastError();
+            err.clear();
+        }
+    }
+    if (on_device) {
         std::vector<gmapf_v2> pts(2 * (size_t)n);
         for (int k = 0; k < n; k++) {
             pts[k] = pos[k];
@@ -556,8 +570,15 @@ int serve_submit(Context& c, const int* ids, const gmapf_v2* pos, int n, const i
             pts[n + k] = a >= 0 && a < c.A ? c.m_pos[a] : pos[k];
         }
         node.resize(pts.size());
-        const int rc = device_locate_points(c, pts.data(), (int)pts.size(), node.data(), err);
-        if (rc) return rc;
+        for (size_t k = 0; k < pts.size(); k += c.dev.loc_cap) {
+            const int m = (int)std::min<size_t>(c.dev.loc_cap, pts.size() - k);
+            if (device_locate_points(c, pts.data() + k, m, node.data() + k, err) != GMAPF_OK) {
+                cudaGetLastError();
+                node.clear();
+                err.clear();
+                break;
+            }
+        }
     }
     for (int k = 0; k < n; k++) {
         const int a = ids[k];

@@ -483,11 +483,11 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
         __syncwarp();
         load_selected();
         if ((lane & 15) == 8 || (lane & 15) == 9) ld_edge_half(p.third, e < 0 ? -1 : e >> 2, c0);
-        c0.info &= ~kEdgeThird;
         // A root's third candidate is in its slot 2, as is one of the other root's when
         // ids outside the navmesh leave a slot empty: by lane, the start's would come
-        // after the target's.  Such a first round goes pass by pass.
-        if ((lane & 14) == 0 && (c0.info & 4u)) c0.info |= kEdgeThird;
+        // after the target's.  Such a candidate is in the second half, marked
+        // (noalloc.cu), and the first round goes pass by pass.
+        if (lane < 2) c0.info &= ~kEdgeThird;
 
         unsigned deg_sum = 0;
         int rounds = 0, expansions = 0, active = 2;  // active: nodes expanded by the coming round

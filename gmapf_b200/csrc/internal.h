@@ -63,7 +63,7 @@ struct __align__(16) EdgeHalf {
     unsigned info;  // its slot as a one-hot bit 0-2, kEdgeThird, and (first half) v's degree from bit 4
     float x, y;
 };
-constexpr unsigned kEdgeThird = 8;  // (first half) there is a third candidate
+constexpr unsigned kEdgeThird = 8;  // (first half) there is a third candidate; (second half) see k_noalloc_rows
 struct __align__(32) EdgeRow {
     EdgeHalf x, y;
 };

@@ -423,9 +423,11 @@ __global__ void __launch_bounds__(256) k_noalloc_rows(const gmapf_node* nodes, i
                 if (q.NeibsIdx[b] == v) back = b;
             const float2 c = node_centroid(nodes, w);
             if (found < 2) {
-                EdgeHalf& h = found == 0 ? o.x : o.y;
+                // (a root's candidate of slot 2 that is not its third: see corridor.cu's first round)
+                const bool late = s == 3 && j == 2;
+                EdgeHalf& h = found == 0 && !late ? o.x : o.y;
                 h.e = w << 2 | back;
-                h.info |= 1u << j;
+                h.info |= late ? 1u << j | kEdgeThird : 1u << j;
                 h.x = c.x;
                 h.y = c.y;
             } else {

@@ -80,6 +80,7 @@ struct DeviceSetup {
     unsigned char* scratch = nullptr;  // device address of g_scratch
     int sms = 0;
     std::unordered_map<int, int> blocks_per_sm;  // (T, C) -> resident one-warp blocks per SM
+    int smem_limit[33] = {};                     // per T: the record form's shared-memory limit
     bool log_ready[33] = {};                     // per T: the log form's kernel has its shared-memory limit
 };
 DeviceSetup g_setup[kMaxDevices];
@@ -473,14 +474,19 @@ cudaError_t run_t(const NoAllocArgs& a, int blocks, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// limit: the kernel's shared-memory limit on the current device, only ever raised
+// (a lower one for a small C would refuse later launches with a larger)
 template <int T>
-int occupancy(int C) {
+int occupancy(int C, int* limit) {
     const size_t smem = smem_per_warp(T, C);
     if (smem > 227 * 1024) return 0;
-    if (cudaFuncSetAttribute(k_search_noalloc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess) {
-        cudaGetLastError();
-        return 0;
+    if ((int)smem > *limit) {
+        if (cudaFuncSetAttribute(k_search_noalloc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        *limit = (int)smem;
     }
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_search_noalloc<T>, 32, smem) != cudaSuccess) {
@@ -490,13 +496,13 @@ int occupancy(int C) {
     return nb;
 }
 
-int occupancy_any(int T, int C) {
+int occupancy_any(int T, int C, int* limit) {
     switch (T) {
-        case 2: return occupancy<2>(C);
-        case 4: return occupancy<4>(C);
-        case 8: return occupancy<8>(C);
-        case 16: return occupancy<16>(C);
-        case 32: return occupancy<32>(C);
+        case 2: return occupancy<2>(C, limit);
+        case 4: return occupancy<4>(C, limit);
+        case 8: return occupancy<8>(C, limit);
+        case 16: return occupancy<16>(C, limit);
+        case 32: return occupancy<32>(C, limit);
         default: return 0;
     }
 }
@@ -572,7 +578,7 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
         const int key = T * 1024 + C;
         auto it = ds->blocks_per_sm.find(key);
         if (it == ds->blocks_per_sm.end()) {
-            it = ds->blocks_per_sm.emplace(key, occupancy_any(T, C)).first;
+            it = ds->blocks_per_sm.emplace(key, occupancy_any(T, C, &ds->smem_limit[T])).first;
             ds->log_ready[T] = ds->log_ready[T] || corridor_full_smem(T);
         }
         per_sm = it->second;

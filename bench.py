@@ -211,7 +211,13 @@ def measured_inst_per_round(T: int, C: int, vm: int):
     return d["inst_per_round"], d["source"]
 
 
-def issue_roofline(rounds: int, search_ms: float, ipr, src, sm_mhz, sms: int):
+def search_kernel(vm: int) -> str:
+    """The kernel that searches the benchmark's maze (long thin corridors) with
+    this visited placement: 2 and 3 are search.cu's only."""
+    return "k_corridor_search" if vm in (1, 4) else "k_search"
+
+
+def issue_roofline(rounds: int, search_ms: float, ipr, src, sm_mhz, sms: int, kernel: str = "k_corridor_search"):
     """The search kernel against the schedulers' issue rate: instructions
     (rounds x instructions per round) per second over 4 schedulers x SMs x SM
     clock (one warp instruction per scheduler per cycle)."""
@@ -220,7 +226,7 @@ def issue_roofline(rounds: int, search_ms: float, ipr, src, sm_mhz, sms: int):
     mhz = sm_mhz or 1965.0
     achieved = rounds * ipr / (search_ms / 1e3) / 1e9
     peak = 4 * sms * mhz / 1e3
-    return {"bound": "issue", "kernel": "k_corridor_search", "achieved": achieved, "peak": peak,
+    return {"bound": "issue", "kernel": kernel, "achieved": achieved, "peak": peak,
             "unit": "G warp instructions/s", "frac": achieved / peak, "inst_per_round": ipr,
             "inst_source": src, "peak_basis": f"4 schedulers x {sms} SMs x {mhz:.0f} MHz (sampled SM clock)"}
 
@@ -885,7 +891,7 @@ def bench_b200(args):
             "e2e_step_ms_over_many_frames": p99_long,
             "e2e_attribution": attribution(wall, parts),
             "e2e_sequential": e2e_seq,
-            "roofline": {"bound": "hbm", "kernel": "k_corridor_search", "achieved": achieved, "peak": peak,
+            "roofline": {"bound": "hbm", "kernel": search_kernel(shape["visited_mode"]), "achieved": achieved, "peak": peak,
                          "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "traffic_source": traffic_src,
                          "search_ms_per_step": statistics.mean(search_ms),
@@ -893,7 +899,7 @@ def bench_b200(args):
                          **search_side_counters(shape["T"], shape["C"], shape["visited_mode"], st_sum["rounds"],
                                                 sum(search_ms))},
             "roofline_issue": issue_roofline(st_sum["rounds"], sum(search_ms), ipr, ipr_src, clocks.get("sm_mhz"),
-                                             sms),
+                                             sms, search_kernel(shape["visited_mode"])),
             "mover": {"maze_frames": moving, "cfg2": cfg2},
             "cpu_baseline": cpu,
             # per frame: target points to the device point location (8 B) and

@@ -321,8 +321,8 @@ __device__ __forceinline__ void walk_path(LG log, int claims, int2* buf, int cap
 // placement 4 a pad so that all but the first warp's share can hold one bitmap
 // -- or, with full_pad, room for one whole bitmap: in a batch with a warp for
 // every request, a search of each block moves its bitmap there while the
-// block's others still run (2,047 searches, 160x160 maze: T=8 25.6 -> 24.0 ms,
-// T=32 10.2 -> 9.6).  In larger batches it would be taken by whichever search
+// block's others still run (2,047 searches, 160x160 maze: T=8 25.6 -> 24.1 ms,
+// T=32 10.2 -> 9.4).  In larger batches it would be taken by whichever search
 // comes first, not by the one that ends the batch (16,384 searches at T=32:
 // 19.0 ms from the start on, 16.9 from the moment no request is left, 16.6 as
 // search.cu does it, once the block's other warps have left).
@@ -876,8 +876,7 @@ __global__ void __launch_bounds__(256, 3) k_corridor_search(SearchParams p, int 
             if (move_plan >= 0) {
                 // shares of warps that have left hold the bitmap from share
                 // `first` on; this warp's queues and frontier move to share `home`
-                // when its own share lies in that run (the deferred items stay in
-                // place in the frontier); the search goes on there
+                // when its own share lies in that run; the search goes on there
                 __threadfence_block();
                 const int first = move_plan & 0xff, home = move_plan >> 8;
                 if (home != wib) {

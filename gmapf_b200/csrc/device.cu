@@ -144,7 +144,7 @@ SceneInfo single_scene(const Context& c) {
 
 // Mover constants of one scene (AgentsMover.h:162,222-224) and its agent grid:
 // cells at least 1.0625 collision distances wide and about one agent per
-// cell (a scan over the cells is part of every moving frame; the collision
+// cell (every moving frame clears their counts; the collision
 // pass reads the 3x3 cells around each agent, so the cell size changes only
 // which agents are read, never the result), at most 2048 per axis; cell ids
 // continue from cell_base.
@@ -652,8 +652,8 @@ int device_start(Context& c, std::string& err) {
     }
     DALLOC(d.cell_of, A);
     DALLOC(d.cell_count, 2 * (size_t)d.cells);
-    DALLOC(d.bucket, 4 * (size_t)d.cells);
-    DALLOC(d.lists, 4 * (size_t)d.cells);
+    DALLOC(d.bucket, 8 * (size_t)d.cells);  // (and the lists' heads)
+    d.lists = d.bucket + 4 * (size_t)d.cells;
     DALLOC(d.next, A);
 
     // pinned host staging

@@ -86,7 +86,7 @@ struct SearchParams {
     int log_bytes;           // placement 1: its entries take 6 bytes (n <= kPackedLogNodes) or 8 (kHalfLogNodes), 0: 16
     int* queues;             // corridor maps: slots x corridor_queue_bytes, or null (queues in shared memory)
     int slots;
-    unsigned* gbm;           // visited mode 3: bm_words 32-bit words per slot, global
+    unsigned* gbm;           // visited placements 3 and 4: bm_words 32-bit words per slot, global
     int* work_ctr;
     int max_rounds;
     int full_pad;            // corridor.cu, visited placement 4: each block has room for one more bitmap
@@ -368,8 +368,8 @@ struct Device {
     int form = 0;            // SearchForm of the sized search
     bool full_pad = false;   // corridor maps, placement 4: room for one more bitmap in each block
     int slots = 0;
-    int vm = 2;                 // visited mode (1, 2 or 3; see launch_search)
-    unsigned* gbm = nullptr;    // visited mode 3: slots x bm_words
+    int vm = 2;                 // visited placement (1 to 4; see launch_search)
+    unsigned* gbm = nullptr;    // visited placements 3 and 4: slots x bm_words
     int bm_words = 0;           // bitmap words per slot
     int rec_cap = 0, log_cap = 0, gbm_cap = 0;  // slots the records / logs / bitmaps hold (kept across reshapes)
     // agent grid

@@ -565,7 +565,7 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
                 cudaGetLastError();
                 return fail(GMAPF_E_CUDA, "cudaDeviceGetAttribute failed");
             }
-            // records start unclaimed: zero them once (query stamps start at 1)
+            // records start unclaimed: zero them once (no query's stamp is 0)
             if (cudaMemsetAsync(ptr, 0, kScratchBytes, s) != cudaSuccess) {
                 cudaGetLastError();
                 return fail(GMAPF_E_CUDA, "clearing the scratch array failed");
@@ -573,8 +573,8 @@ extern "C" gmapf_status gmapf_search_batch_noalloc(const gmapf_node* d_nodes, in
             ds->scratch = static_cast<unsigned char*>(ptr);
             ds->ready = true;
         }
-        // the kernel attribute and occupancy query run once per (T, C) on
-        // this device; later calls make no CUDA calls besides the launch
+        // the kernel attributes and occupancy query run once per (T, C) on this
+        // device; later calls only launch (one to three kernels and at most one clear)
         const int key = T * 1024 + C;
         auto it = ds->blocks_per_sm.find(key);
         if (it == ds->blocks_per_sm.end()) {

@@ -41,7 +41,6 @@ __device__ __forceinline__ void ld_edge_row(const EdgeRow* rows, int k, EdgeHalf
     ld_edge_half(&rows->x, k < 0 ? -1 : 2 * (long long)k + 1, y);
 }
 
-// the row into shared memory, asynchronously; copies_done waits for this thread's copies
 // a word through L2, 0 (and no access) without `on`
 __device__ __forceinline__ unsigned ld_word_if(const unsigned* p, bool on) {
     unsigned w;
@@ -52,7 +51,8 @@ __device__ __forceinline__ unsigned ld_word_if(const unsigned* p, bool on) {
     return w;
 }
 
-// (k < 0: zeros, and nothing is read)
+// the row into shared memory, asynchronously (k < 0: zeros, and nothing is read);
+// copies_done waits for this thread's copies
 __device__ __forceinline__ void copy_edge_row(EdgeHalf* to, const EdgeRow* rows, int k) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(to);
     const EdgeRow* from = rows + max(k, 0);

@@ -11,7 +11,8 @@
 //     released;
 //   - each poll launches the queries admitted since the previous launch as a
 //     micro-batch on one of kStreams streams that is idle; every stream owns
-//     its own range of search slots, so up to kStreams batches run at once
+//     its own range of search slots (a burst takes idle neighbours' ranges
+//     too), so up to kStreams batches run at once
 //     and queries that arrive while others run start without waiting for
 //     them (a persistent launch over its batch: warps take queries as they
 //     free up);
@@ -454,8 +455,8 @@ int serve_start(Context& c, int max_in_flight, std::string& err) {
         return GMAPF_E_CAPACITY;
     }
     const double per_slot = (double)search_slot_bytes(n, d.vm, d.bm_words, d.form, c.T, c.C);
-    // the drain launch is persistent while queries keep coming: leave one
-    // block per SM for the frames' own kernels
+    // batches may fill all slots for as long as their longest search: leave one
+    // block's share of every SM to the frames' kernels (small blocks, see launch_compact)
     const int drain_per_sm = per_sm > 1 ? per_sm - 1 : 1;
     sv.room = per_sm > 1;
     long long slots = std::min<long long>((long long)sms * drain_per_sm * gpb, (long long)(0.25 * freeb / per_slot));

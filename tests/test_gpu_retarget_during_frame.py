@@ -1,0 +1,38 @@
+"""A bulk retarget during a running frame does not wait for the frame's searches."""
+import time
+
+import numpy as np
+import pytest
+
+import gmapf_b200 as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,Cap", [(8, 32), (32, 16)])
+def test_bulk_retarget_during_a_frame(T, Cap):
+    # 5,000 searches of some ten thousand rounds each fill the GPU; the points
+    # of the next targets are located beside them
+    from test_gpu_frame_kernels import inside, winding_map
+    nodes = winding_map(100, 100, 8.0)
+    rng = np.random.default_rng(T)
+    A = 5000
+    g = G.GMAPF()
+    g.Init(G.make_config(A, 0.1, 1.0, A, T, Cap))
+    g.FillMapManually(nodes)
+    for p in inside(nodes[:200], A, rng):
+        g.AddAgent(p)
+    ids = np.arange(A, dtype=np.int32)
+    g.ManualStart()
+    for _ in range(3):  # (the first frame records its graph, the first call makes its buffers)
+        g.set_targets(ids, inside(nodes[-200:], A, rng))
+        goal = inside(nodes[-200:], A, rng)
+        g.AsyncStep(0.01)
+        time.sleep(0.001)  # the searches run
+        t0 = time.perf_counter()
+        g.set_targets(ids, goal)
+        t1 = time.perf_counter()
+        running = not g.step_ready()
+        g.WaitStepEnd()
+        t2 = time.perf_counter()
+    assert running and t1 - t0 < t2 - t1

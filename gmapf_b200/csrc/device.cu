@@ -270,14 +270,17 @@ int pick_slots(Context& c, int& blocks, long long& budget, std::string& err) {
     long long best_slots = 0;
     const int want_vm = c.opt.visited_mode ? c.opt.visited_mode : c.tuned_vm;
     const int want_bt = c.opt.block_threads ? c.opt.block_threads : c.tuned_bt;
-    auto consider = [&](int vm, int bt, int form) {  // true: it has room for a block
+    auto slots_of = [&](int vm, int bt, int form) -> long long {  // 0: no room for a block
         const int per_sm = search_max_blocks_per_sm(c.T, c.C, bt, vm, d.bm_words, form);
-        if (per_sm <= 0) return false;
+        if (per_sm <= 0) return 0;
         const int gpb = bt / 32;  // one request slot per warp
-        long long slots = std::min((long long)sms * per_sm * gpb,
-                                   budget / (long long)search_slot_bytes(n, vm, d.bm_words, form, c.T, c.C));
-        slots = (slots / gpb) * gpb;
-        if (slots < gpb) return false;
+        const long long slots = std::min((long long)sms * per_sm * gpb,
+                                         budget / (long long)search_slot_bytes(n, vm, d.bm_words, form, c.T, c.C));
+        return (slots / gpb) * gpb;
+    };
+    auto consider = [&](int vm, int bt, int form) {  // true: it has room for a block
+        const long long slots = slots_of(vm, bt, form);
+        if (slots == 0) return false;
         const long long weight = form != FORM_RECORDS ? (vm == 1 ? 64 : 40) : (vm == 1 ? 40 : vm >= 3 ? 30 : 20);
         long long score = 10 * slots * weight + (vm == 4 ? 1 : 0);
         if (form == FORM_LOG_GLOBAL) score = score * 9 / 10;
@@ -306,6 +309,20 @@ int pick_slots(Context& c, int& blocks, long long& budget, std::string& err) {
             log = std::any_of(bts.begin(), bts.end(), [&](int bt) {
                 return search_max_blocks_per_sm(c.T, c.C, bt, vm, d.bm_words, FORM_RECORDS) > 0;
             });
+        // The plain form serves a frame's requests in chunks of the slots, one after the
+        // other, and a chunk takes as long as its longest search: search.cu's kernel
+        // where its slots (T = 8: 4,144 against 3,552) save more than a fifth of the chunks
+        // (4,000 requests on the 24x24 maze, T=8: one chunk 0.86 ms, two of corridor.cu's
+        // kernel 1.26; 16,000: four 3.25, five 3.23).
+        if (log && c.opt.mode == GMAPF_MODE_PLAIN) {
+            long long rec = 0, logs = 0;
+            for (int bt : bts) {
+                rec = std::max(rec, slots_of(vm, bt, FORM_RECORDS));
+                logs = std::max({logs, slots_of(vm, bt, FORM_LOG), slots_of(vm, bt, FORM_LOG_GLOBAL)});
+            }
+            const long long P = std::max(1, c.cfg.PathFinderParallelAgents);
+            if (rec > 0 && logs > 0) log = 5 * ((P + rec - 1) / rec) >= 4 * ((P + logs - 1) / logs);
+        }
         bool placed = false;
         if (log)
             for (int bt : bts)

@@ -71,3 +71,22 @@ def test_search_memory_within_its_budget(options):
         return used
 
     assert held(budget) - held(1 << 20) <= budget + (8 << 20)  # (2 MiB granules)
+
+
+@pytest.mark.parametrize("P,one_chunk", [(3000, True), (4000, True), (16384, False)])
+def test_plain_form_takes_the_kernel_with_fewer_chunks(oracle_mod, P, one_chunk):
+    # T=8: search.cu's kernel has 28 warps per SM (4,144 slots), corridor.cu's 24 (3,552)
+    nodes = long_strip(2700)
+    g = G.GMAPF()
+    g.Init(G.make_config(1, 2.0, 1.0, P, 8, 32))
+    g.set_options(mode=G.MODE_PLAIN)
+    g.FillMapManually(nodes)
+    g.ManualStart()
+    assert (g.search_shape()["slots"] >= P) == one_chunk
+    rng = np.random.default_rng(P)
+    s, t = (rng.integers(0, len(nodes), 300).astype(np.int32) for _ in range(2))
+    f, l, p, _ = g.search_batch(s, t, len(nodes))
+    of, ol, op, _ = oracle_mod.OMap(nodes).search_batch(s, t, 8, 32)
+    assert np.array_equal(f, of) and np.array_equal(l, ol)
+    for i in np.nonzero(f)[0]:
+        assert np.array_equal(p[i, :l[i]], op[i, :l[i]])

@@ -23,19 +23,8 @@ def no_room_of_its_own(lib, n, T, Cap, threads):
                for q in (False, True))
 
 
-@pytest.mark.parametrize("T,Cap,threads,n", [(8, 32, 64, 90_000), (8, 32, 128, 126_000), (32, 16, 64, 90_000),
-                                             (32, 16, 128, 140_000), (32, 16, 256, 180_000), (2, 4, 256, 270_000)])
-def test_move_into_finished_warps_shares(lib, oracle_mod, T, Cap, threads, n):
-    from test_gpu_placements import long_strip
-    nodes = long_strip(n)
-    g = G.GMAPF()
-    g.Init(G.make_config(1, 2.0, 1.0, 1, T, Cap))
-    g.set_options(visited_mode=4, block_threads=threads, promote_rounds=1)
-    g.FillMapManually(nodes)
-    g.ManualStart()
-    shape = g.search_shape()
-    assert shape["visited_mode"] == 4 and shape["block_threads"] == threads
-    assert no_room_of_its_own(lib, n, T, Cap, threads)
+def compare(oracle_mod, g, nodes, T, Cap):
+    n, shape = len(nodes), g.search_shape()
     om = oracle_mod.OMap(nodes)
     rng = np.random.default_rng(n)
     for q in (shape["slots"] // 2, shape["slots"] + 700):
@@ -52,3 +41,35 @@ def test_move_into_finished_warps_shares(lib, oracle_mod, T, Cap, threads, n):
             assert np.array_equal(p[i, :l[i]], op[i, :l[i]]), f"path {i} differs"
         for k in ("rounds", "expansions", "claims", "deg_sum"):
             assert st[k] == ost[k], k
+
+
+def started(nodes, T, Cap, **options):
+    g = G.GMAPF()
+    g.Init(G.make_config(1, 2.0, 1.0, 1, T, Cap))
+    g.set_options(visited_mode=4, promote_rounds=1, **options)
+    g.FillMapManually(nodes)
+    g.ManualStart()
+    assert g.search_shape()["visited_mode"] == 4
+    return g
+
+
+@pytest.mark.parametrize("T,Cap,threads,n", [(8, 32, 64, 90_000), (8, 32, 128, 126_000), (32, 16, 64, 90_000),
+                                             (32, 16, 128, 140_000), (32, 16, 256, 180_000), (2, 4, 256, 270_000)])
+def test_move_into_finished_warps_shares(lib, oracle_mod, T, Cap, threads, n):
+    from test_gpu_placements import long_strip
+    nodes = long_strip(n)
+    g = started(nodes, T, Cap, block_threads=threads)
+    assert g.search_shape()["block_threads"] == threads
+    assert no_room_of_its_own(lib, n, T, Cap, threads)
+    compare(oracle_mod, g, nodes, T, Cap)
+
+
+@pytest.mark.parametrize("T,Cap", [(8, 32), (32, 16)])
+def test_room_of_its_own(lib, oracle_mod, T, Cap):
+    # the same batches where every block has room for a bitmap of its own: taken
+    # while the block's others run, and by the tail of a batch that the queue feeds
+    from test_gpu_placements import long_strip
+    n = 30_000
+    g = started(long_strip(n), T, Cap, block_threads=256)
+    assert not no_room_of_its_own(lib, n, T, Cap, 256)
+    compare(oracle_mod, g, long_strip(n), T, Cap)
